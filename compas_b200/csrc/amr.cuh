@@ -284,26 +284,28 @@ __device__ void amr_face_flux(const double* U, const Grid& g, int d, int i, int 
                 wR[n] = weno5_f32(P[1][n], P[2][n], P[3][n], P[4][n], P[5][n], -1);
             }
         }
-#pragma unroll
-        for (int n = 0; n < N; ++n) {
-            WfL[n] = wL[n];
-            WfR[n] = wR[n];
-        }
-        M::prim2cons(UL, WfL, e, err);
-        M::prim2cons(UR, WfR, e, err);
         if constexpr (NPH) {
-            if constexpr (SCHEME != 6) if (SCHEME != 2 || code != 11) {
-                M::consistent_limit(UL, P[2], 1, dxd, 1, e, err);
-                M::consistent_limit(UR, P[3], 1, dxd, -1, e, err);
+            auto general = [&](const double* ul, const double* ur) {
+                riemann<M>(id_riemann, F, fnc, cm, ul, ur, e, d, id_k, err);
+            };
+            if (SCHEME == 5 || (SCHEME == 2 && code != 11))
+                nphase_mixed_face<M, true>(F, fnc, cm, wL, wR, P[2], P[3], 1, dxd, e, d, id_k, SCHEME == 5 && id_riemann == 2,
+                                           general, err);
+            else
+                nphase_mixed_face<M, false>(F, fnc, cm, wL, wR, P[2], P[3], 1, dxd, e, d, id_k, SCHEME == 6 && id_riemann == 2,
+                                            general, err);
+        } else if constexpr (SXN) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                WfL[n] = wL[n];
+                WfR[n] = wR[n];
             }
+            M::prim2cons(UL, WfL, e, err);
+            M::prim2cons(UR, WfR, e, err);
             riemann<M>(id_riemann, F, fnc, cm, UL, UR, e, d, id_k, err);
-        } else if (id_riemann != 2) {
-            float cmf;
-            llf_hll_mixed<M>(id_riemann, F, fnc, cmf, UL, UR, wL, wR, e, d, id_k);
         } else {
             float cmf;
-            if constexpr (M::KIND == kModelFive) fiveeq_hllc_mixed<D>(F, fnc, cmf, UL, UR, wL, wR, e, d, id_k);
-            else sixeq_hllc_mixed<D>(F, fnc, cmf, UL, UR, wL, wR, e, d);
+            mixed_riemann<M>(id_riemann, F, fnc, cmf, wL, wR, e, d, id_k, MixedState<M>{wL, wR, e});
         }
     }
 }

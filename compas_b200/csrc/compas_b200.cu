@@ -223,7 +223,7 @@ struct StepParams {
     int dts_cap;
 };
 
-__global__ void step_begin_kernel(StepCtl* s, StepParams p) {
+__device__ __forceinline__ void step_begin(StepCtl* s, StepParams p) {
     if (s->done) return;
     if (!(s->t < s->stop_time)) {
         s->done = 1;
@@ -248,10 +248,28 @@ __global__ void step_begin_kernel(StepCtl* s, StepParams p) {
     if (p.dts && s->steps < p.dts_cap) p.dts[s->steps] = dt0;
 }
 
+__global__ void step_begin_kernel(StepCtl* s, StepParams p) { step_begin(s, p); }
+
 __global__ void step_end_kernel(StepCtl* s) {
     if (s->done) return;
     s->t += s->dt;
     s->steps += 1;
+}
+
+// The start of a level step in one launch: the ghost cells of the state, and beside them ComputeDt and the
+// step's t += dt (no stage reads t), which as launches of their own took about 3 and 2 us of a step.
+__global__ void step_begin_fill_kernel(StepCtl* s, StepParams p, BcArgs a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        step_begin(s, p);
+        if (!s->done) {
+            s->t += s->dt;
+            s->steps += 1;
+        }
+    }
+    const long long total = ghost_count(a.g);
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
+         q += (long long)gridDim.x * blockDim.x)
+        fill_ghost_cell(a.U, a.g, a.N, a.D, a.m0, a.lo, a.hi, q);
 }
 
 __global__ void set_time_kernel(StepCtl* s, double t0, double stop_time, int reset) {
@@ -314,6 +332,8 @@ static Eos make_eos(const compas_b200_parm* p) {
     e.fA1 = (float)p->A1; e.fA2 = (float)p->A2;
     e.fB1 = (float)p->B1; e.fB2 = (float)p->B2;
     e.fC1 = (float)p->C1; e.fC2 = (float)p->C2;
+    e.fG1 = (float)(p->A1 + 1.0); e.fG2 = (float)(p->A2 + 1.0);
+    e.fiA1 = (float)(1.0 / p->A1); e.fiA2 = (float)(1.0 / p->A2);
     return e;
 }
 
@@ -473,7 +493,7 @@ static int launch_list(int physics, int dim, int nphase, int limiter, int precis
     return COMPAS_B200_OK;
 }
 
-static int launch_fill(const compas_b200_parm* p, const compas_b200_geom* geo, double* U, cudaStream_t st) {
+static BcArgs bc_args(const compas_b200_parm* p, const compas_b200_geom* geo, double* U) {
     BcArgs b;
     b.U = U;
     b.g = make_grid(p, geo);
@@ -484,13 +504,18 @@ static int launch_fill(const compas_b200_parm* p, const compas_b200_geom* geo, d
         b.lo[d] = geo->lo_bc[d];
         b.hi[d] = geo->hi_bc[d];
     }
-    const Grid& g = b.g;
-    const long long total = 2LL * g.gz * g.pxy + 2LL * g.ng * g.px * g.n[2] + 2LL * g.ng * g.n[1] * g.n[2];
+    return b;
+}
+
+static unsigned fill_blocks(long long cells, int threads) {
+    const long long blocks = (cells + threads - 1) / threads;
+    return (unsigned)std::max(1LL, std::min(blocks, 148LL * 16));
+}
+
+static int launch_fill(const compas_b200_parm* p, const compas_b200_geom* geo, double* U, cudaStream_t st) {
+    const BcArgs b = bc_args(p, geo, U);
     const int threads = 256;
-    long long blocks = (total + threads - 1) / threads;
-    if (blocks > 148LL * 16) blocks = 148LL * 16;
-    if (blocks < 1) blocks = 1;
-    fill_boundary_kernel<<<(unsigned)blocks, threads, 0, st>>>(b);
+    fill_boundary_kernel<<<fill_blocks(ghost_count(b.g), threads), threads, 0, st>>>(b);
     CUDA_TRY(cudaGetLastError());
     return COMPAS_B200_OK;
 }
@@ -498,23 +523,11 @@ static int launch_fill(const compas_b200_parm* p, const compas_b200_geom* geo, d
 // The ghost cells of the slab l0 <= l < l1 (fill_boundary_slab_kernel).
 static int launch_fill_slab(const compas_b200_parm* p, const compas_b200_geom* geo, double* U, int l0, int l1,
                             cudaStream_t st) {
-    BcArgs b;
-    b.U = U;
-    b.g = make_grid(p, geo);
-    b.N = nstate(p);
-    b.D = p->dim;
-    b.m0 = mom0_of(p->physics, p->nphase);
-    for (int d = 0; d < 3; ++d) {
-        b.lo[d] = geo->lo_bc[d];
-        b.hi[d] = geo->hi_bc[d];
-    }
+    const BcArgs b = bc_args(p, geo, U);
     const long long unit = (p->dim == 3) ? b.g.pxy : b.g.px;
     const long long total = (long long)(l1 - l0) * unit;
     const int threads = 256;
-    long long blocks = (total + threads - 1) / threads;
-    if (blocks > 148LL * 16) blocks = 148LL * 16;
-    if (blocks < 1) blocks = 1;
-    fill_boundary_slab_kernel<<<(unsigned)blocks, threads, 0, st>>>(b, l0, l1);
+    fill_boundary_slab_kernel<<<fill_blocks(total, threads), threads, 0, st>>>(b, l0, l1);
     CUDA_TRY(cudaGetLastError());
     return COMPAS_B200_OK;
 }
@@ -596,12 +609,21 @@ static int tune_candidates(F&& launch, cudaStream_t st, int reps, TuneChoice* be
     return rc;
 }
 
+// The launch shape of a box that nothing has tuned: a box of fewer tiles than the GPU has SMs takes the shape
+// with one large CTA per tile (a 64^2 FIVEEQS WENO5 FP64 stage, 16 tiles: shape 0 / 1 see kern_impl.cuh).
+static int default_shape(const compas_b200_parm* p, const compas_b200_geom* g) {
+    const int ts = (p->dim == 2) ? kTile2 : kTile3;
+    const long long tiles = (long long)((g->n[0] + ts - 1) / ts) * ((g->n[1] + ts - 1) / ts) *
+                            (p->dim == 3 ? (g->n[2] + ts - 1) / ts : 1);
+    return (p->id_limiter >= 5 && !p->thinc && tiles <= 148) ? 1 : 0;
+}
+
 // The tuned launch shape / tile order of a single box of this size, if a level has tuned it in this
 // process (the drop-in entry points reuse it; they never time anything themselves).
 static int cached_shape(const compas_b200_parm* p, const compas_b200_geom* g, StageArgs& a) {
-    if (!p->autotune) return 0;
     TuneChoice c;
-    if (!tune_lookup(tune_key(p, "box", g->n[0], g->n[1], p->dim == 3 ? g->n[2] : 1), &c)) return 0;
+    if (!p->autotune || !tune_lookup(tune_key(p, "box", g->n[0], g->n[1], p->dim == 3 ? g->n[2] : 1), &c))
+        return default_shape(p, g);
     a.order = c.order;
     return c.shape;
 }
@@ -675,6 +697,10 @@ static StageArgs base_args(const compas_b200_parm* p, const compas_b200_geom* g)
     a.pf_phasic = (p->pf_phase2flux == 0);
     a.muscl = p->id_weno ? (p->id_limiter == 3 ? 10 : (p->id_limiter == 4 ? 11 : -1)) : p->id_limiter;
     a.pf_hll = (p->pf_flux == 1);
+    for (int d = 0; d < 3; ++d) {
+        a.lo_bc[d] = g->lo_bc[d];
+        a.hi_bc[d] = g->hi_bc[d];
+    }
     a.thinc.use_normal = p->thinc_use_normal;
     a.thinc.eps = p->thinc_eps;
     a.thinc.beta = p->thinc_beta;
@@ -1520,7 +1546,7 @@ int compas_b200_rk3_step_noalloc(const compas_b200_parm* p, const compas_b200_ge
     double* U2 = reinterpret_cast<double*>(base + kNoAllocHeadBytes + kNoAllocStateBytes);
     cudaStream_t st = (cudaStream_t)stream;
     // the scratch keeps the previous call's contents: dt is rewritten here, U1 and U2 are fully
-    // written (valid cells by the stage kernels, ghosts by the boundary fill) before they are read
+    // written (valid cells by the stage kernels) before they are read
     noalloc_set_dt_kernel<<<1, 1, 0, st>>>(dt_dev, dt);
     CUDA_TRY(cudaGetLastError());
     StageArgs a = base_args(p, g);
@@ -1532,7 +1558,9 @@ int compas_b200_rk3_step_noalloc(const compas_b200_parm* p, const compas_b200_ge
     double* ins[3] = {U, U1, U2};
     double* outs[3] = {U1, U2, U};
     for (int s = 0; s < 3; ++s) {
-        if ((rc = launch_fill(p, g, ins[s], st))) return rc;
+        // the scratch states' ghost cells are read through the boundary conditions (THINC reads them in memory)
+        a.map_ghosts = s > 0 && !p->thinc;
+        if (!a.map_ghosts && (rc = launch_fill(p, g, ins[s], st))) return rc;
         a.stage = s;
         a.Us = ins[s];
         a.U0 = U;
@@ -1667,6 +1695,11 @@ static int tune_level(compas_b200_level* lv, cudaStream_t st) {
         a.err = reinterpret_cast<unsigned int*>(scratch + 2);
         auto launch = [&](int sh, int od, int tm) {
             a.order = od;
+            // the TMA form needs the boundary fill that the others do without
+            if (tm) {
+                const int rc = launch_fill(&lv->p, &lv->g, lv->U, st);
+                if (rc) return rc;
+            }
             return launch_stage(&lv->p, a, st, 0, sh, tm ? &lv->maps[0] : nullptr);
         };
         const int rc = tune_candidates(launch, st, 2, &c, lv->maps[0].valid ? 2 : 1);
@@ -1682,7 +1715,6 @@ static int tune_level(compas_b200_level* lv, cudaStream_t st) {
     return COMPAS_B200_OK;
 }
 
-// The launches of one coarse step: ComputeDt, then three (fill, stage) pairs, then t += dt.
 static StepParams level_step_params(const compas_b200_level* lv) {
     StepParams sp;
     sp.cfl = lv->p.cfl;
@@ -1696,11 +1728,19 @@ static StepParams level_step_params(const compas_b200_level* lv) {
     return sp;
 }
 
+// Whether the stage kernels of the level read the ghost cells of the intermediate states through the boundary
+// conditions instead of from a boundary fill: all but the THINC and TMA variants, which read them in memory.
+static bool maps_ghosts(const compas_b200_level* lv) { return !lv->p.thinc && !lv->use_tma; }
+
+static int step_launches(const compas_b200_level* lv) { return maps_ghosts(lv) ? 4 : 6; }
+
+// The launches of one coarse step: ComputeDt with the ghost cells of U, then the three stages.
 static int enqueue_step(compas_b200_level* lv, cudaStream_t st) {
     const compas_b200_parm* p = &lv->p;
     const compas_b200_geom* g = &lv->g;
-    const StepParams sp = level_step_params(lv);
-    step_begin_kernel<<<1, 1, 0, st>>>(lv->ctl, sp);
+    const BcArgs bc = bc_args(p, g, lv->U);
+    const int threads = 256;
+    step_begin_fill_kernel<<<fill_blocks(ghost_count(bc.g), threads), threads, 0, st>>>(lv->ctl, level_step_params(lv), bc);
     CUDA_TRY(cudaGetLastError());
     StageArgs a = base_args(p, g);
     a.mode = kModeStage;
@@ -1712,16 +1752,16 @@ static int enqueue_step(compas_b200_level* lv, cudaStream_t st) {
     double* bufs_out[3] = {lv->U1, lv->U2, lv->U};
     int rc;
     a.order = lv->order;
+    const bool map = maps_ghosts(lv);
     for (int s = 0; s < 3; ++s) {
-        if ((rc = launch_fill(p, g, bufs_in[s], st))) return rc;
+        if (s > 0 && !map && (rc = launch_fill(p, g, bufs_in[s], st))) return rc;
+        a.map_ghosts = s > 0 && map;
         a.stage = s;
         a.Us = bufs_in[s];
         a.U0 = lv->U;
         a.Uout = bufs_out[s];
         if ((rc = launch_stage(p, a, st, 0, lv->shape, lv->use_tma ? &lv->maps[s] : nullptr))) return rc;
     }
-    step_end_kernel<<<1, 1, 0, st>>>(lv->ctl);
-    CUDA_TRY(cudaGetLastError());
     return COMPAS_B200_OK;
 }
 
@@ -1854,7 +1894,7 @@ int compas_b200_level_advance(compas_b200_level* lv, int nsteps, double stop_tim
             a.mode = kModeCmax;
             a.cmax = &lv->ctl->cmax;
             a.err = &lv->ctl->err;
-            if ((rc = launch_stage(&lv->p, a, st))) return rc;
+            if ((rc = launch_stage(&lv->p, a, st, 0, default_shape(&lv->p, &lv->g)))) return rc;
         }
         lv->launches += 2;
         lv->need_init = false;
@@ -1873,7 +1913,7 @@ int compas_b200_level_advance(compas_b200_level* lv, int nsteps, double stop_tim
         // a Phase-Field step of the same dt; its host loop reads dt, max|u| and max|grad Q|.
         for (int s = 0; s < nsteps; ++s) {
             if ((rc = enqueue_step(lv, st))) return rc;
-            lv->launches += 8;
+            lv->launches += step_launches(lv);
             StepCtl h;
             CUDA_TRY(cudaMemcpyAsync(&h, lv->ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, st));
             CUDA_TRY(cudaStreamSynchronize(st));
@@ -1921,7 +1961,7 @@ int compas_b200_level_advance(compas_b200_level* lv, int nsteps, double stop_tim
         for (int s = 0; s < nsteps; ++s)
             if ((rc = enqueue_step(lv, st))) return rc;
     }
-    lv->launches += 8LL * nsteps;
+    lv->launches += (long long)step_launches(lv) * nsteps;
     return COMPAS_B200_OK;
 }
 
@@ -2339,10 +2379,13 @@ static int batch_enqueue_step(compas_b200_batch* b, cudaStream_t st) {
     const int N = nstate_of(b->physics, b->dim, b->nphase);
     int rc;
     for (int s = 0; s < 3; ++s) {
-        FillListArgs F{b->d_boxes, b->d_nbox, b->d_ghost_off, N, b->dim, mom0_of(b->physics, b->nphase), s};
-        fill_list_kernel<<<148 * 8, 256, 0, st>>>(F);
-        CUDA_TRY(cudaGetLastError());
-        ListArgs L{b->d_boxes, b->d_nbox, b->d_tile_off, kModeStage, s, b->order};
+        // the intermediate states' ghost cells are read through the boundary conditions
+        if (s == 0) {
+            FillListArgs F{b->d_boxes, b->d_nbox, b->d_ghost_off, N, b->dim, mom0_of(b->physics, b->nphase), s};
+            fill_list_kernel<<<148 * 8, 256, 0, st>>>(F);
+            CUDA_TRY(cudaGetLastError());
+        }
+        ListArgs L{b->d_boxes, b->d_nbox, b->d_tile_off, kModeStage, s, b->order, s > 0};
         if ((rc = launch_list(b->physics, b->dim, b->nphase, b->limiter, b->precision, L, st, b->shape))) return rc;
     }
     step_end_list_kernel<<<4, 256, 0, st>>>(b->d_ctl, b->d_slots, b->d_nbox);
@@ -2391,7 +2434,7 @@ int compas_b200_batch_advance(compas_b200_batch* b, int nsteps, int use_graph, v
         for (int s = 0; s < nsteps; ++s)
             if ((rc = batch_enqueue_step(b, st))) return rc;
     }
-    b->launches += 8LL * nsteps;
+    b->launches += 6LL * nsteps;
     return COMPAS_B200_OK;
 }
 

@@ -10,65 +10,77 @@
 
 namespace compas {
 
-// Launch shapes of the stage kernel (threads per CTA, CTAs per SM) among which the autotuner picks;
+// Launch shapes of the stage kernels (threads per CTA, CTAs per SM) among which the autotuner picks;
 // the tile is 8^3 in 3D and 16^2 in 2D for every shape. The register budget is set per SM
-// sub-partition (16384 registers each, warps dealt round-robin): in 3D, 6 warps at 2 CTAs/SM get
-// 168 registers per thread, 8 warps 128, 9 warps 112; in 2D, 272 threads at 2 CTAs/SM get 96, at 1
-// CTA/SM 232, 136 threads at 4 CTAs/SM 120. Every shape covers the 576 (3D) or 272 (2D) faces of a
-// direction in whole rounds or nearly so. Shape 0 is the default when tuning is off.
-template <int D, int S>
+// sub-partition (16384 registers each, warps dealt round-robin). Shape 0 is the default where nothing is
+// tuned, shape 1 that of boxes of fewer tiles than SMs (default_shape in compas_b200.cu).
+//
+// stage_tile (FACES = false): its passes have 512 (3D) or 18 x 16 x components (2D) reconstruction items and
+// 576 or 272 faces, so 288 threads fill both nearly evenly. B200, us per stage, shapes 0 / 1 / 2:
+// 96^3 SIXEQS WENO5 mixed 250 / 266 / 285, FP64 793 / 810 / 888; 1024 x 512 FIVEEQS WENO5B mixed
+// 87 / 125 / 95, FP64 260 / 324 / 298; 128^2 FIVEEQS WENO5 FP64 (64 tiles) 68 / 58 / 82.
+// stage_tile_faces (FACES = true): 576 (3D) or 272 (2D) faces a direction and one thread each.
+template <bool FACES, int D, bool MIX, int S>
 struct ShapeParams;
-template <> struct ShapeParams<3, 0> { static constexpr int NT = 192, MINB = 2; };
-template <> struct ShapeParams<3, 1> { static constexpr int NT = 256, MINB = 2; };
-template <> struct ShapeParams<3, 2> { static constexpr int NT = 288, MINB = 2; };
-template <> struct ShapeParams<2, 0> { static constexpr int NT = 272, MINB = 2; };
-template <> struct ShapeParams<2, 1> { static constexpr int NT = 272, MINB = 1; };
-template <> struct ShapeParams<2, 2> { static constexpr int NT = 136, MINB = 4; };
+template <bool MIX> struct ShapeParams<false, 3, MIX, 0> { static constexpr int NT = 288, MINB = 2; };
+template <bool MIX> struct ShapeParams<false, 3, MIX, 1> { static constexpr int NT = 576, MINB = 1; };
+template <> struct ShapeParams<false, 3, true, 2> { static constexpr int NT = 192, MINB = 2; };
+template <> struct ShapeParams<false, 3, false, 2> { static constexpr int NT = 384, MINB = 1; };
+template <> struct ShapeParams<false, 2, true, 0> { static constexpr int NT = 144, MINB = 4; };
+template <> struct ShapeParams<false, 2, true, 2> { static constexpr int NT = 288, MINB = 2; };
+template <> struct ShapeParams<false, 2, false, 0> { static constexpr int NT = 288, MINB = 2; };
+template <> struct ShapeParams<false, 2, false, 2> { static constexpr int NT = 144, MINB = 4; };
+template <bool MIX> struct ShapeParams<false, 2, MIX, 1> { static constexpr int NT = 512, MINB = 1; };
+template <bool MIX> struct ShapeParams<true, 3, MIX, 0> { static constexpr int NT = 192, MINB = 2; };
+template <bool MIX> struct ShapeParams<true, 3, MIX, 1> { static constexpr int NT = 256, MINB = 2; };
+template <bool MIX> struct ShapeParams<true, 3, MIX, 2> { static constexpr int NT = 288, MINB = 2; };
+template <bool MIX> struct ShapeParams<true, 2, MIX, 0> { static constexpr int NT = 272, MINB = 2; };
+template <bool MIX> struct ShapeParams<true, 2, MIX, 1> { static constexpr int NT = 272, MINB = 1; };
+template <bool MIX> struct ShapeParams<true, 2, MIX, 2> { static constexpr int NT = 136, MINB = 4; };
 
-template <class M, int S = 0>
+template <class M, bool FACES, bool MIX, int S>
 struct LaunchShape {
     static constexpr int TS = (M::D == 2) ? kTile2 : kTile3;
     static constexpr int TZ = (M::D == 2) ? 1 : TS;
-    static constexpr int NT = ShapeParams<M::D, S>::NT;
-    static constexpr int MINB = ShapeParams<M::D, S>::MINB;
+    static constexpr int NT = ShapeParams<FACES, M::D, MIX, S>::NT;
+    static constexpr int MINB = ShapeParams<FACES, M::D, MIX, S>::MINB;
 };
 
 // One CTA per tile of the box.
 template <class M, int SCHEME, bool MIX, int VAR, int SH>
 static cudaError_t launch_stage_v(const StageArgs& a, cudaStream_t st) {
-    using S = LaunchShape<M, SH>;
-    using T = TileShape<M, S::TS, S::TS, S::TZ, typename std::conditional<MIX, float, double>::type, false,
-                        VAR == kVarPhaseField>;
+    using S = LaunchShape<M, SCHEME == 2 || VAR == kVarThinc, MIX, SH>;
+    constexpr size_t SMEM = tile_smem<M, SCHEME, MIX, VAR, S::TS, S::TZ, S::MINB>();
     auto kern = stage_kernel<M, SCHEME, MIX, VAR, S::TS, S::TS, S::TZ, S::NT, S::MINB>;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
     const long long tiles = a.tile_count > 0 ? (long long)a.tile_count
                                              : (long long)((a.g.n[0] + S::TS - 1) / S::TS) *
                                                    ((a.g.n[1] + S::TS - 1) / S::TS) * ((a.g.n[2] + S::TZ - 1) / S::TZ);
-    kern<<<(unsigned)tiles, S::NT, T::SMEM, st>>>(a);
+    kern<<<(unsigned)tiles, S::NT, SMEM, st>>>(a);
     return cudaGetLastError();
 }
 
 // One box with the y/z halo slabs staged by TMA (3D mixed form; the maps describe a.Us).
 template <class M, int SCHEME, int SH>
 static cudaError_t launch_stage_tma(const StageArgs& a, const TmaMaps& tm, cudaStream_t st) {
-    using S = LaunchShape<M, SH>;
-    using T = TileShape<M, S::TS, S::TS, S::TZ, float, true>;
+    using S = LaunchShape<M, false, true, SH>;
+    constexpr size_t SMEM = tile_smem<M, SCHEME, true, kVarTma, S::TS, S::TZ, S::MINB>();
     auto kern = stage_kernel_tma<M, SCHEME, true, S::TS, S::TS, S::TZ, S::NT, S::MINB>;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
     const long long tiles = a.tile_count > 0 ? (long long)a.tile_count
                                              : (long long)((a.g.n[0] + S::TS - 1) / S::TS) *
                                                    ((a.g.n[1] + S::TS - 1) / S::TS) * ((a.g.n[2] + S::TZ - 1) / S::TZ);
-    kern<<<(unsigned)tiles, S::NT, T::SMEM, st>>>(a, tm);
+    kern<<<(unsigned)tiles, S::NT, SMEM, st>>>(a, tm);
     return cudaGetLastError();
 }
 
@@ -120,20 +132,20 @@ static cudaError_t launch_stage_m(const KernelChoice& k, const StageArgs& a, cud
 // Persistent box-list launch: one resident wave of CTAs walks the tiles of every box.
 template <class M, int SCHEME, bool MIX, int SH>
 static cudaError_t launch_list_v(const ListArgs& L, cudaStream_t st) {
-    using S = LaunchShape<M, SH>;
-    using T = TileShape<M, S::TS, S::TS, S::TZ, typename std::conditional<MIX, float, double>::type>;
+    using S = LaunchShape<M, SCHEME == 2, MIX, SH>;
+    constexpr size_t SMEM = tile_smem<M, SCHEME, MIX, kVarPlain, S::TS, S::TZ, S::MINB>();
     auto kern = stage_list_kernel<M, SCHEME, MIX, S::TS, S::TS, S::TZ, S::NT, S::MINB>;
     static int grid = 0;
     if (!grid) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
         if (e != cudaSuccess) return e;
         int dev = 0, sms = 0, per = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, S::NT, T::SMEM)) != cudaSuccess) return e;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, S::NT, SMEM)) != cudaSuccess) return e;
         grid = sms * std::max(per, 1);
     }
-    kern<<<grid, S::NT, T::SMEM, st>>>(L);
+    kern<<<grid, S::NT, SMEM, st>>>(L);
     return cudaGetLastError();
 }
 

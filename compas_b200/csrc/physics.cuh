@@ -42,6 +42,20 @@ __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b 
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double sgn0(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0); }
 
+// FP32 reciprocal and square root of the mixed form, one instruction each (both within about one unit in
+// the last place; subnormal inputs read as 0). Callers keep their arguments away from the subnormal range.
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float sqrt_ftz(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Reciprocal for the mixed-precision form: an FP32 estimate refined by one Newton-Raphson step for
 // 1/x, r1 = r0 (2 - x r0), evaluated in FP64 (Newton's method; the relative error squares, from
 // about 2^-22 to below 2^-43). For x of FP32 range (densities, A_P). The quantities scaled by it are
@@ -66,6 +80,7 @@ struct Eos {
     // FP32 copies (round to nearest) of A, B, C of the two phases for the mixed form's FP32 wave speeds,
     // so that the face loop converts no coefficients
     float fA1, fA2, fB1, fB2, fC1, fC2;
+    float fG1, fG2, fiA1, fiA2;  // A + 1 and 1/A
 };
 
 // Model families of the stage kernel (the M::KIND of each model struct).
@@ -197,6 +212,29 @@ struct FiveEq {
         U[IA] = alpha1;
     }
 
+    // Conserved state of FP32 face primitives in FP64 (the mixed form).
+    __device__ static __forceinline__ void prim2cons_f32(double* U, const float* W, const Eos& e) {
+        const double a1r1 = W[0], a2r2 = W[1], p = W[IE], alpha1 = W[IA];
+        const double rho = a1r1 + a2r2;
+        const double alpha2 = 1.0 - alpha1;
+        const double phi1 = (e.C1 > 0.0) ? alpha1 - e.C1 * a1r1 : alpha1;
+        const double phi2 = (e.C2 > 0.0) ? alpha2 - e.C2 * a2r2 : alpha2;
+        const double AP = fma(phi1, e.A1, phi2 * e.A2);
+        const double BP = fma(phi1, e.B1, phi2 * e.B2);
+        const double rho_D = fma(a1r1, e.D1, a2r2 * e.D2);
+        double u[D], k = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            u[d] = W[2 + d];
+            k = fma(u[d], u[d], k);
+            U[2 + d] = rho * u[d];
+        }
+        U[0] = a1r1;
+        U[1] = a2r2;
+        U[IE] = fma(0.5 * rho, k, fma(AP, p, BP) + rho_D);
+        U[IA] = alpha1;
+    }
+
     // THINC side of a face: the face state Uf (MUSCL-minmod) with its volume fraction replaced by the
     // THINC value af; phase densities, velocity and pressure are kept, masses, momentum and energy
     // rebuilt (Reconstruct_State_From_VolumeFraction,
@@ -292,9 +330,6 @@ struct FiveEq {
     __device__ static __forceinline__ void hllc_uw(double* Fout, double* fnc, double& cmax, const double* UL,
                                                    const double* WL, const double* UR, const double* WR, const Eos& e,
                                                    int d, int id_k, unsigned int* err) {
-        double FL[N], FR[N];
-        flux(FL, UL, WL, d);
-        flux(FR, UR, WR, d);
         const double cL = sound_speed(WL, e, id_k, err);
         const double cR = sound_speed(WR, e, id_k, err);
         const double VL = pick<D>(WL + 2, d), VR = pick<D>(WR + 2, d);
@@ -309,26 +344,41 @@ struct FiveEq {
         const double rhoR = WR[0] + WR[1];
         const double S_Star = (((pR - pL) + (rhoL * VL) * (SL - VL)) - (rhoR * VR) * (SR - VR)) /
                               (rhoL * (SL - VL) - rhoR * (SR - VR));
-        const double s = sgn0(S_Star);
-        const double hp = 0.5 * (1.0 + s), hm = 0.5 * (1.0 - s);
-        const double fL = (SL - VL) / (SL - S_Star);
-        const double fR = (SR - VR) / (SR - S_Star);
-        // normal face velocity: Vel[d] = hp*uL_d + hm*uR_d, then += hp*Sm*(fL-1) + hm*Sp*(fR-1)
-        double vel = hp * VL + hm * VR;
-        vel = vel + ((hp * Sm) * (fL - 1.0) + (hm * Sp) * (fR - 1.0));
-        fnc[0] = vel;
+        // The reference blends both sides' star states with the weights (1 + sign S*)/2 and (1 - sign S*)/2; a
+        // side of weight 0 adds nothing, so only the upwind one is formed, and both where S* is 0 (or NaN).
+        const bool left = S_Star > 0.0, both = !(left || S_Star < 0.0);
+        auto side = [&](bool lt, double* F, double& vel, double& dvel) {
+            const double V = lt ? VL : VR, p = lt ? pL : pR, rho = lt ? rhoL : rhoR, SK = lt ? SL : SR;
+            const double Sb = lt ? Sm : Sp;
+            double U[N], W[N];
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            double sL = fL * UL[i];
-            double sR = fR * UR[i];
-            if (i == 2 + d) {
-                sL = sL + (fL * rhoL) * (S_Star - VL);
-                sR = sR + (fR * rhoR) * (S_Star - VR);
-            } else if (i == IE) {
-                sL = sL + (fL * (S_Star - VL)) * (rhoL * S_Star + pL / (SL - VL));
-                sR = sR + (fR * (S_Star - VR)) * (rhoR * S_Star + pR / (SR - VR));
+            for (int i = 0; i < N; ++i) {
+                U[i] = lt ? UL[i] : UR[i];
+                W[i] = lt ? WL[i] : WR[i];
             }
-            Fout[i] = hp * (FL[i] + Sm * (sL - UL[i])) + hm * (FR[i] + Sp * (sR - UR[i]));
+            flux(F, U, W, d);
+            const double f = (SK - V) / (SK - S_Star);
+            vel = V;
+            dvel = f - 1.0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                double star = f * U[i];
+                if (i == 2 + d) star = star + (f * rho) * (S_Star - V);
+                else if (i == IE) star = star + (f * (S_Star - V)) * (rho * S_Star + p / (SK - V));
+                F[i] = F[i] + Sb * (star - U[i]);
+            }
+        };
+        double v, dv;
+        side(left || both, Fout, v, dv);
+        // normal face velocity: Vel[d] = hp*uL_d + hm*uR_d, then += hp*Sm*(fL-1) + hm*Sp*(fR-1)
+        if (both) {
+            double F[N], vr, dvr;
+            side(false, F, vr, dvr);
+#pragma unroll
+            for (int i = 0; i < N; ++i) Fout[i] = 0.5 * Fout[i] + 0.5 * F[i];
+            fnc[0] = (0.5 * v + 0.5 * vr) + ((0.5 * Sm) * dv + (0.5 * Sp) * dvr);
+        } else {
+            fnc[0] = v + (left ? Sm : Sp) * dv;
         }
         const double qL = cL + sqrt(ksum<D>(WL + 2));
         const double qR = cR + sqrt(ksum<D>(WR + 2));
@@ -348,25 +398,26 @@ __device__ __forceinline__ float fiveeq_c_f32(const float* w, const Eos& e, int 
     using M = FiveEq<DIM>;
     constexpr int IE = M::IE, IA = M::IA;
     const float p = w[IE], a1 = w[IA], a2 = 1.0f - a1;
-    const float A1 = e.fA1, A2 = e.fA2, B1 = e.fB1, B2 = e.fB2;
-    const float r1 = __fdividef(__fmaf_rn(A1 + 1.0f, p, B1), A1);
-    const float r2 = __fdividef(__fmaf_rn(A2 + 1.0f, p, B2), A2);
+    const float r1 = __fmaf_rn(e.fG1, p, e.fB1);  // A_k rho_k c_k^2
+    const float r2 = __fmaf_rn(e.fG2, p, e.fB2);
     const float ph1 = (e.fC1 > 0.0f) ? a1 - e.fC1 * w[0] : a1;
     const float ph2 = (e.fC2 > 0.0f) ? a2 - e.fC2 * w[1] : a2;
-    float rc2;
+    const float rho = w[0] + w[1];
+    float rc2;  // c^2
     if (id_k == 0)
-        rc2 = __fdividef(__fmaf_rn(a1 * A1, r1, (a2 * A2) * r2), __fmaf_rn(ph1, A1, ph2 * A2));
+        rc2 = __fmaf_rn(a1, r1, a2 * r2) * rcp_ftz(__fmaf_rn(ph1, e.fA1, ph2 * e.fA2) * rho);
     else
-        rc2 = __fdividef(1.0f, __fdividef(ph1, r1) + __fdividef(ph2, r2));
-    return sqrtf(fmaxf(rc2, 0.0f) / (w[0] + w[1]));
+        rc2 = rcp_ftz(__fmaf_rn(ph1 * e.fA1, rcp_ftz(r1), (ph2 * e.fA2) * rcp_ftz(r2)) * rho);
+    return sqrt_ftz(fmaxf(rc2, 0.0f));
 }
 
-template <int DIM>
-__device__ __forceinline__ void fiveeq_hllc_mixed(double* Fout, double* fnc, float& cmax, const double* UL,
-                                                  const double* UR, const float* wL, const float* wR,
-                                                  const Eos& e, int d, int id_k) {
+// `state(left, U)` gives the conserved state of the left (true) or right face state; only the upwind one
+// is asked for (both where S* is exactly 0).
+template <int DIM, class State>
+__device__ __forceinline__ void fiveeq_hllc_mixed(double* Fout, double* fnc, float& cmax, const float* wL,
+                                                  const float* wR, const Eos& e, int d, int id_k, State state) {
     using M = FiveEq<DIM>;
-    constexpr int N = M::N, IE = M::IE, IA = M::IA;
+    constexpr int N = M::N, IE = M::IE;
     const float cL = fiveeq_c_f32<DIM>(wL, e, id_k), cR = fiveeq_c_f32<DIM>(wR, e, id_k);
     const float VL = (d == 0) ? wL[2] : ((d == 1 || DIM == 2) ? wL[3] : wL[DIM == 3 ? 4 : 3]);
     const float VR = (d == 0) ? wR[2] : ((d == 1 || DIM == 2) ? wR[3] : wR[DIM == 3 ? 4 : 3]);
@@ -374,67 +425,43 @@ __device__ __forceinline__ void fiveeq_hllc_mixed(double* Fout, double* fnc, flo
     const float rhoL = wL[0] + wL[1], rhoR = wR[0] + wR[1];
     const float Va = 0.5f * (VL + VR), ca = 0.5f * (cL + cR);
     const float SL = fminf(Va - ca, VL - cL), SR = fmaxf(Va + ca, VR + cR);
-    const float Sm = fminf(0.0f, SL), Sp = fmaxf(0.0f, SR);
     // delta form: dS = S* - V and f - 1 from the jumps, exactly 0 where p and V are uniform
     const float gL = SL - VL, gR = SR - VR;
     const float aL = rhoL * gL, aR = rhoR * gR;
-    const float inv_den = __fdividef(1.0f, aL - aR);
+    const float inv_den = rcp_ftz(aL - aR);
     const float dp = pR - pL, dV = VL - VR;
     const float dSL = __fmaf_rn(aR, dV, dp) * inv_den, dSR = __fmaf_rn(aL, dV, dp) * inv_den;
     const float S = VL + dSL;
-    const float fm1L = __fdividef(dSL, gL - dSL), fm1R = __fdividef(dSR, gR - dSR);
-    const float eL = (1.0f + fm1L) * dSL * (rhoL * S + __fdividef(pL, gL));
-    const float eR = (1.0f + fm1R) * dSR * (rhoR * S + __fdividef(pR, gR));
-    const float mL = (1.0f + fm1L) * rhoL * dSL, mR = (1.0f + fm1R) * rhoR * dSR;
-    if (S != 0.0f) {
-        // FP64 assembly of the upwind side K only (left where S > 0): F = F_K + S_K (U*_K - U_K), the
-        // value of the blend below, whose weights are then 1 and 0
-        const bool lt = (S > 0.0f);
-        const double V = lt ? VL : VR, p = lt ? pL : pR, gm = lt ? fm1L : fm1R, Sk = lt ? Sm : Sp;
-        const double en = lt ? eL : eR, mo = lt ? mL : mR;
+    // F = F_K + S_K (U*_K - U_K) of the upwind side K (left where S* > 0) from its conserved state u: with
+    // c = V + S_K (f - 1) every transported component is u c, plus the pressure terms
+    auto side = [&](bool lt, double* F, double& vel) {
+        const float Vf = lt ? VL : VR, pf = lt ? pL : pR, rho = lt ? rhoL : rhoR, g = lt ? gL : gR, dS = lt ? dSL : dSR;
+        const float Sf = lt ? fminf(0.0f, SL) : fmaxf(0.0f, SR);
+        const float fm1 = dS * rcp_ftz(g - dS), f = 1.0f + fm1;
+        const float enf = f * dS * __fmaf_rn(rho, S, pf * rcp_ftz(g)), mof = f * rho * dS;
+        const double V = Vf, p = pf, Sk = Sf;
+        const double c = fma(Sk, (double)fm1, V);
+        double u[N];
+        state(lt, u);
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const double u = lt ? UL[i] : UR[i];
-            double f = u * V, dd = gm * u;
-            if (i == IE) {
-                f = (u + p) * V;
-                dd += en;
-            } else if (i >= 2 && i < 2 + DIM && i - 2 == d) {
-                f += p;
-                dd += mo;
-            }
-            Fout[i] = fma(Sk, dd, f);
-        }
-        fnc[0] = fma(Sk, gm, V);
-    } else {
-    const float s = 0.0f;
-    // FP64 assembly: F = h+ (F_L + S- (U*_L - U_L)) + h- (F_R + S+ (U*_R - U_R))
-    const double hp = 0.5 * (1.0 + s), hm = 0.5 * (1.0 - s);
-    const double gmL = fm1L, gmR = fm1R, Smd = Sm, Spd = Sp;
-    const double VLd = VL, VRd = VR, pLd = pL, pRd = pR;
+        for (int i = 0; i < N; ++i) F[i] = u[i] * c;
+        const double mo = fma(Sk, (double)mof, p);
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        double fl = UL[i] * VLd, fr = UR[i] * VRd;
-        double dL = gmL * UL[i], dR = gmR * UR[i];
-        if (i == IE) {
-            fl = (UL[IE] + pLd) * VLd;
-            fr = (UR[IE] + pRd) * VRd;
-            dL += (double)eL;
-            dR += (double)eR;
-        } else if (i >= 2 && i < 2 + DIM && i - 2 == d) {
-            fl += pLd;
-            fr += pRd;
-            dL += (double)mL;
-            dR += (double)mR;
-        }
-        Fout[i] = hp * (fl + Smd * dL) + hm * (fr + Spd * dR);
+        for (int i = 0; i < DIM; ++i) F[2 + i] = (i == d) ? F[2 + i] + mo : F[2 + i];
+        F[IE] = F[IE] + fma(Sk, (double)enf, p * V);
+        vel = c;
+    };
+    side(S >= 0.0f, Fout, fnc[0]);
+    if (S == 0.0f) {  // the mean of both sides
+        double F[N], v;
+        side(false, F, v);
+#pragma unroll
+        for (int i = 0; i < N; ++i) Fout[i] = 0.5 * (Fout[i] + F[i]);
+        fnc[0] = 0.5 * (fnc[0] + v);
     }
-    fnc[0] = (hp * VLd + hm * VRd) + ((hp * Smd) * gmL + (hm * Spd) * gmR);
-    }
-    float kL = wL[2] * wL[2] + wL[3] * wL[3], kR = wR[2] * wR[2] + wR[3] * wR[3];
-    if (DIM == 3) { kL += wL[4] * wL[4]; kR += wR[4] * wR[4]; }
-    cmax = fmaxf(cL + sqrtf(kL), cR + sqrtf(kR));
-    (void)IA;
+    float kL = __fmaf_rn(wL[2], wL[2], wL[3] * wL[3]), kR = __fmaf_rn(wR[2], wR[2], wR[3] * wR[3]);
+    if (DIM == 3) { kL = __fmaf_rn(wL[4], wL[4], kL); kR = __fmaf_rn(wR[4], wR[4], kR); }
+    cmax = fmaxf(cL + sqrt_ftz(kL), cR + sqrt_ftz(kR));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -524,6 +551,26 @@ struct SixEq {
         U[IA] = alpha1;
     }
 
+    // Conserved state of FP32 face primitives in FP64 (the mixed form).
+    __device__ static __forceinline__ void prim2cons_f32(double* U, const float* W, const Eos& e) {
+        const double a1r1 = W[0], a2r2 = W[1], alpha1 = W[IA], alpha2 = 1.0 - alpha1;
+        const double rho = a1r1 + a2r2;
+        double k = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            const double u = W[2 + d];
+            k = fma(u, u, k);
+            U[2 + d] = rho * u;
+        }
+        k = 0.5 * k;
+        const double xi1 = nasg_xi(alpha1, a1r1, e.C1, nullptr), xi2 = nasg_xi(alpha2, a2r2, e.C2, nullptr);
+        U[0] = a1r1;
+        U[1] = a2r2;
+        U[IE1] = fma(a1r1, e.D1 + k, fma(e.A1 * xi1, (double)W[IE1], (xi1 * alpha1) * e.B1));
+        U[IE2] = fma(a2r2, e.D2 + k, fma(e.A2 * xi2, (double)W[IE2], (xi2 * alpha2) * e.B2));
+        U[IA] = alpha1;
+    }
+
     // THINC side of a face (include/Operators_Compressible6Eq/FVM_Reconstruction2Face_Conservative_THINC_K_Compressible6Eq.H:14-62):
     // phase densities, velocity and phase pressures of the face state are kept.
     __device__ static __forceinline__ void thinc_rebuild(double* Uo, const double* Uf, double af, const Eos& e,
@@ -590,9 +637,6 @@ struct SixEq {
     __device__ static __forceinline__ void hllc_uw(double* Fout, double* fnc, double& cmax, const double* UL,
                                                    const double* WL, const double* UR, const double* WR, const Eos& e,
                                                    int d, int /*id_k*/, unsigned int* err) {
-        double FL[N], FR[N];
-        flux(FL, UL, WL, d);
-        flux(FR, UR, WR, d);
         const double cL = sound_speed(WL, e, err);
         const double cR = sound_speed(WR, e, err);
         const double VL = pick<D>(WL + 2, d), VR = pick<D>(WR + 2, d);
@@ -600,54 +644,60 @@ struct SixEq {
         const double SR = dmax(VL + cL, VR + cR);
         const double Sm = dmin(0.0, SL);
         const double Sp = dmax(0.0, SR);
-        const double a1r1L = WL[0], a2r2L = WL[1], a1r1R = WR[0], a2r2R = WR[1];
-        const double a1p1L = WL[IE1], a2p2L = WL[IE2], a1p1R = WR[IE1], a2p2R = WR[IE2];
-        const double rhoL = a1r1L + a2r2L;
-        const double rhoR = a1r1R + a2r2R;
-        const double pL = a1p1L + a2p2L;
-        const double pR = a1p1R + a2p2R;
+        const double rhoL = WL[0] + WL[1];
+        const double rhoR = WR[0] + WR[1];
+        const double pL = WL[IE1] + WL[IE2];
+        const double pR = WR[IE1] + WR[IE2];
         const double S_Star = (((pR - pL) + (rhoL * VL) * (SL - VL)) - (rhoR * VR) * (SR - VR)) /
                               (rhoL * (SL - VL) - rhoR * (SR - VR));
-        const double fL = (SL - VL) / (SL - S_Star);
-        const double fR = (SR - VR) / (SR - S_Star);
-        const double a1r1Ls = fL * a1r1L, a1r1Rs = fR * a1r1R;
-        const double a2r2Ls = fL * a2r2L, a2r2Rs = fR * a2r2R;
-        double UsL[N], UsR[N];
-        UsL[0] = a1r1Ls; UsL[1] = a2r2Ls;
-        UsR[0] = a1r1Rs; UsR[1] = a2r2Rs;
+        // the upwind side's star state, and both where S* is 0 (FiveEq::hllc_uw)
+        const bool left = S_Star > 0.0, both = !(left || S_Star < 0.0);
+        auto side = [&](bool lt, double* F, double* nc, double& dvel) {
+            const double V = lt ? VL : VR, rho = lt ? rhoL : rhoR, SK = lt ? SL : SR, Sb = lt ? Sm : Sp;
+            double U[N], W[N];
 #pragma unroll
-        for (int c = 0; c < D; ++c) {
-            const double uLc = WL[2 + c], uRc = WR[2 + c];
-            const double nrm = (c == d) ? 1.0 : 0.0;
-            UsL[2 + c] = (fL * rhoL) * (uLc + nrm * (S_Star - uLc));
-            UsR[2 + c] = (fR * rhoR) * (uRc + nrm * (S_Star - uRc));
+            for (int i = 0; i < N; ++i) {
+                U[i] = lt ? UL[i] : UR[i];
+                W[i] = lt ? WL[i] : WR[i];
+            }
+            flux(F, U, W, d);
+            const double f = (SK - V) / (SK - S_Star);
+            const double a1r1 = W[0], a2r2 = W[1], a1p1 = W[IE1], a2p2 = W[IE2];
+            const double a1r1s = f * a1r1, a2r2s = f * a2r2;
+            F[0] = F[0] + Sb * (a1r1s - U[0]);
+            F[1] = F[1] + Sb * (a2r2s - U[1]);
+#pragma unroll
+            for (int c = 0; c < D; ++c) {
+                const double u = W[2 + c];
+                const double nrm = (c == d) ? 1.0 : 0.0;
+                F[2 + c] = F[2 + c] + Sb * ((f * rho) * (u + nrm * (S_Star - u)) - U[2 + c]);
+            }
+            const double a1p1s = (a1p1 + ((V - SK) * a1r1) * V) - ((S_Star - SK) * a1r1s) * S_Star;
+            const double a2p2s = (a2p2 + ((V - SK) * a2r2) * V) - ((S_Star - SK) * a2r2s) * S_Star;
+            const double E1 = (((V - SK) * U[IE1] + V * a1p1) - S_Star * a1p1s) / (S_Star - SK);
+            const double E2 = (((V - SK) * U[IE2] + V * a2p2) - S_Star * a2p2s) / (S_Star - SK);
+            F[IE1] = F[IE1] + Sb * (E1 - U[IE1]);
+            F[IE2] = F[IE2] + Sb * (E2 - U[IE2]);
+            F[IA] = F[IA] + Sb * (f * W[IA] - U[IA]);
+            // normal components of Vel (its two terms), Vel*a1p1, Vel*a2p2
+            nc[0] = V;
+            dvel = f - 1.0;
+            nc[1] = V * a1p1 + (1.0 * Sb) * (V * a1p1 - S_Star * a1p1s) / (S_Star - SK);
+            nc[2] = V * a2p2 + (1.0 * Sb) * (V * a2p2 - S_Star * a2p2s) / (S_Star - SK);
+        };
+        double dv;
+        side(left || both, Fout, fnc, dv);
+        if (both) {
+            double F[N], nc[3], dvr;
+            side(false, F, nc, dvr);
+#pragma unroll
+            for (int i = 0; i < N; ++i) Fout[i] = 0.5 * Fout[i] + 0.5 * F[i];
+            fnc[0] = (0.5 * fnc[0] + 0.5 * nc[0]) + ((0.5 * Sm) * dv + (0.5 * Sp) * dvr);
+            fnc[1] = 0.5 * fnc[1] + 0.5 * nc[1];
+            fnc[2] = 0.5 * fnc[2] + 0.5 * nc[2];
+        } else {
+            fnc[0] = fnc[0] + (left ? Sm : Sp) * dv;
         }
-        const double a1p1Ls = (a1p1L + ((VL - SL) * a1r1L) * VL) - ((S_Star - SL) * a1r1Ls) * S_Star;
-        const double a1p1Rs = (a1p1R + ((VR - SR) * a1r1R) * VR) - ((S_Star - SR) * a1r1Rs) * S_Star;
-        const double a2p2Ls = (a2p2L + ((VL - SL) * a2r2L) * VL) - ((S_Star - SL) * a2r2Ls) * S_Star;
-        const double a2p2Rs = (a2p2R + ((VR - SR) * a2r2R) * VR) - ((S_Star - SR) * a2r2Rs) * S_Star;
-        UsL[IE1] = (((VL - SL) * UL[IE1] + VL * a1p1L) - S_Star * a1p1Ls) / (S_Star - SL);
-        UsR[IE1] = (((VR - SR) * UR[IE1] + VR * a1p1R) - S_Star * a1p1Rs) / (S_Star - SR);
-        UsL[IE2] = (((VL - SL) * UL[IE2] + VL * a2p2L) - S_Star * a2p2Ls) / (S_Star - SL);
-        UsR[IE2] = (((VR - SR) * UR[IE2] + VR * a2p2R) - S_Star * a2p2Rs) / (S_Star - SR);
-        UsL[IA] = fL * WL[IA];
-        UsR[IA] = fR * WR[IA];
-        const double s = sgn0(S_Star);
-        const double hp = 0.5 * (1.0 + s), hm = 0.5 * (1.0 - s);
-        // normal components of Vel, Vel*a1p1, Vel*a2p2
-        const double uLd = VL, uRd = VR;
-        double vel = hp * uLd + hm * uRd;
-        vel = vel + ((hp * Sm) * (fL - 1.0) + (hm * Sp) * (fR - 1.0));
-        const double va1 = hp * (uLd * a1p1L + (1.0 * Sm) * (VL * a1p1L - S_Star * a1p1Ls) / (S_Star - SL)) +
-                           hm * (uRd * a1p1R + (1.0 * Sp) * (VR * a1p1R - S_Star * a1p1Rs) / (S_Star - SR));
-        const double va2 = hp * (uLd * a2p2L + (1.0 * Sm) * (VL * a2p2L - S_Star * a2p2Ls) / (S_Star - SL)) +
-                           hm * (uRd * a2p2R + (1.0 * Sp) * (VR * a2p2R - S_Star * a2p2Rs) / (S_Star - SR));
-        fnc[0] = vel;
-        fnc[1] = va1;
-        fnc[2] = va2;
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            Fout[i] = hp * (FL[i] + Sm * (UsL[i] - UL[i])) + hm * (FR[i] + Sp * (UsR[i] - UR[i]));
         const double qL = cL + sqrt(ksum<D>(WL + 2));
         const double qR = cR + sqrt(ksum<D>(WR + 2));
         cmax = dmax(qL, qR);
@@ -661,184 +711,195 @@ template <int DIM>
 __device__ __forceinline__ float sixeq_c_f32(const float* w, const Eos& e) {
     using M = SixEq<DIM>;
     constexpr int IE1 = M::IE1, IE2 = M::IE2, IA = M::IA;
-    const float a1 = w[IA];
-    const float xi1 = (e.fC1 > 0.0f && a1 > 0.0f) ? 1.0f - e.fC1 * __fdividef(w[0], a1) : 1.0f;
-    const float xi2 = (e.fC2 > 0.0f && 1.0f - a1 > 0.0f) ? 1.0f - e.fC2 * __fdividef(w[1], 1.0f - a1) : 1.0f;
-    const float r1 = __fdividef(__fmaf_rn(e.fA1 + 1.0f, w[IE1], a1 * e.fB1), e.fA1 * xi1);
-    const float r2 = __fdividef(__fmaf_rn(e.fA2 + 1.0f, w[IE2], (1.0f - a1) * e.fB2), e.fA2 * xi2);
-    return sqrtf(fmaxf(r1 + r2, 0.0f) / (w[0] + w[1]));
+    const float a1 = w[IA], a2 = 1.0f - a1;
+    float r1 = __fmaf_rn(e.fG1, w[IE1], a1 * e.fB1) * e.fiA1;
+    float r2 = __fmaf_rn(e.fG2, w[IE2], a2 * e.fB2) * e.fiA2;
+    if (e.fC1 > 0.0f && a1 > 0.0f) r1 *= rcp_ftz(1.0f - e.fC1 * (w[0] * rcp_ftz(a1)));
+    if (e.fC2 > 0.0f && a2 > 0.0f) r2 *= rcp_ftz(1.0f - e.fC2 * (w[1] * rcp_ftz(a2)));
+    return sqrt_ftz(fmaxf(r1 + r2, 0.0f) * rcp_ftz(w[0] + w[1]));
 }
 
-template <int DIM>
-__device__ __forceinline__ void sixeq_hllc_mixed(double* Fout, double* fnc, float& cmax, const double* UL,
-                                                 const double* UR, const float* wL, const float* wR,
-                                                 const Eos& e, int d) {
+template <int DIM, class State>
+__device__ __forceinline__ void sixeq_hllc_mixed(double* Fout, double* fnc, float& cmax, const float* wL,
+                                                 const float* wR, const Eos& e, int d, State state) {
     using M = SixEq<DIM>;
-    constexpr int N = M::N, IE1 = M::IE1, IE2 = M::IE2, IA = M::IA;
+    constexpr int N = M::N, IE1 = M::IE1, IE2 = M::IE2;
     const float cL = sixeq_c_f32<DIM>(wL, e), cR = sixeq_c_f32<DIM>(wR, e);
     const float VL = (d == 0) ? wL[2] : ((d == 1 || DIM == 2) ? wL[3] : wL[DIM == 3 ? 4 : 3]);
     const float VR = (d == 0) ? wR[2] : ((d == 1 || DIM == 2) ? wR[3] : wR[DIM == 3 ? 4 : 3]);
     const float SL = fminf(VL - cL, VR - cR), SR = fmaxf(VL + cL, VR + cR);
-    const float Sm = fminf(0.0f, SL), Sp = fmaxf(0.0f, SR);
     const float rhoL = wL[0] + wL[1], rhoR = wR[0] + wR[1];
     const float pL = wL[IE1] + wL[IE2], pR = wR[IE1] + wR[IE2];
     // delta form: dS = S* - V and f - 1 from the jumps, exactly 0 where p and V are uniform
     const float gL = SL - VL, gR = SR - VR;
     const float aL = rhoL * gL, aR = rhoR * gR;
-    const float inv_den = __fdividef(1.0f, aL - aR);
+    const float inv_den = rcp_ftz(aL - aR);
     const float dp = pR - pL, dV = VL - VR;
     const float dSL = __fmaf_rn(aR, dV, dp) * inv_den, dSR = __fmaf_rn(aL, dV, dp) * inv_den;
     const float S = VL + dSL;
-    const float qL = __fdividef(dSL, gL - dSL), qR = __fdividef(dSR, gR - dSR);  // f - 1
-    const float fL = 1.0f + qL, fR = 1.0f + qR;
-    // phase pressures at the star state: (alpha p)* = alpha p + alpha rho (S - V) dS, and the
-    // pressure part t of the phase-energy star state E* = f E + t, t = dS ((alpha p) + S* alpha rho g)/(g - dS)
-    const float a1p1L = wL[IE1], a2p2L = wL[IE2], a1p1R = wR[IE1], a2p2R = wR[IE2];
-    const float tL1 = qL * __fmaf_rn(S * wL[0], gL, a1p1L), tR1 = qR * __fmaf_rn(S * wR[0], gR, a1p1R);
-    const float tL2 = qL * __fmaf_rn(S * wL[1], gL, a2p2L), tR2 = qR * __fmaf_rn(S * wR[1], gR, a2p2R);
-    const float mL = fL * rhoL * dSL, mR = fR * rhoR * dSR;
-    if (S != 0.0f) {
-        // FP64 assembly of the upwind side K only (left where S > 0): F = F_K + S_K (U*_K - U_K), the
-        // value of the blend below, whose weights are then 1 and 0
-        const bool lt = (S > 0.0f);
-        const double V = lt ? VL : VR, gm = lt ? qL : qR, Sk = lt ? Sm : Sp;
-        const double p1 = lt ? a1p1L : a1p1R, p2 = lt ? a2p2L : a2p2R;
-        const double mo = lt ? mL : mR, t1 = lt ? tL1 : tR1, t2 = lt ? tL2 : tR2;
+    // the upwind side as in fiveeq_hllc_mixed; phase pressures at the star state (alpha p)* = alpha p + alpha rho
+    // (S - V) dS, and the pressure part t of the phase-energy star state E* = f E + t,
+    // t = dS ((alpha p) + S* alpha rho g)/(g - dS)
+    auto side = [&](bool lt, double* F, double* nc) {
+        const float Vf = lt ? VL : VR, rho = lt ? rhoL : rhoR, g = lt ? gL : gR, dS = lt ? dSL : dSR;
+        const float p1f = lt ? wL[IE1] : wR[IE1], p2f = lt ? wL[IE2] : wR[IE2];
+        const float r1 = lt ? wL[0] : wR[0], r2 = lt ? wL[1] : wR[1];
+        const float Sf = lt ? fminf(0.0f, SL) : fmaxf(0.0f, SR);
+        const float q = dS * rcp_ftz(g - dS);  // f - 1
+        const float t1f = q * __fmaf_rn(S * r1, g, p1f), t2f = q * __fmaf_rn(S * r2, g, p2f);
+        const float mof = (1.0f + q) * rho * dS;
+        const double V = Vf, p1 = p1f, p2 = p2f, Sk = Sf;
+        const double c = fma(Sk, (double)q, V);
+        double u[N];
+        state(lt, u);
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const double u = lt ? UL[i] : UR[i];
-            double f = u * V, dd = gm * u;
-            if (i >= 2 && i < 2 + DIM && i - 2 == d) {
-                f += p1 + p2;
-                dd += mo;
-            } else if (i == IE1) {
-                f = (u + p1) * V;
-                dd += t1;
-            } else if (i == IE2) {
-                f = (u + p2) * V;
-                dd += t2;
-            }
-            Fout[i] = fma(Sk, dd, f);
-        }
-        fnc[0] = fma(Sk, gm, V);
-        fnc[1] = fma(Sk, t1, V * p1);
-        fnc[2] = fma(Sk, t2, V * p2);
-    } else {
-    const float s = 0.0f;
-    const double hp = 0.5 * (1.0 + s), hm = 0.5 * (1.0 - s);
-    const double gmL = qL, gmR = qR, Smd = Sm, Spd = Sp;
-    const double VLd = VL, VRd = VR;
-    const double p1L = a1p1L, p2L = a2p2L, p1R = a1p1R, p2R = a2p2R;
+        for (int i = 0; i < N; ++i) F[i] = u[i] * c;
+        const double mo = fma(Sk, (double)mof, p1 + p2);
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        double fl = UL[i] * VLd, fr = UR[i] * VRd;
-        double dL = gmL * UL[i], dR = gmR * UR[i];
-        if (i >= 2 && i < 2 + DIM && i - 2 == d) {
-            fl += p1L + p2L;
-            fr += p1R + p2R;
-            dL += (double)mL;
-            dR += (double)mR;
-        } else if (i == IE1) {
-            fl = (UL[IE1] + p1L) * VLd;
-            fr = (UR[IE1] + p1R) * VRd;
-            dL += (double)tL1;
-            dR += (double)tR1;
-        } else if (i == IE2) {
-            fl = (UL[IE2] + p2L) * VLd;
-            fr = (UR[IE2] + p2R) * VRd;
-            dL += (double)tL2;
-            dR += (double)tR2;
-        }
-        Fout[i] = hp * (fl + Smd * dL) + hm * (fr + Spd * dR);
+        for (int i = 0; i < DIM; ++i) F[2 + i] = (i == d) ? F[2 + i] + mo : F[2 + i];
+        nc[0] = c;
+        nc[1] = fma(Sk, (double)t1f, V * p1);
+        nc[2] = fma(Sk, (double)t2f, V * p2);
+        F[IE1] = F[IE1] + nc[1];
+        F[IE2] = F[IE2] + nc[2];
+    };
+    side(S >= 0.0f, Fout, fnc);
+    if (S == 0.0f) {  // the mean of both sides
+        double F[N], nc[3];
+        side(false, F, nc);
+#pragma unroll
+        for (int i = 0; i < N; ++i) Fout[i] = 0.5 * (Fout[i] + F[i]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) fnc[i] = 0.5 * (fnc[i] + nc[i]);
     }
-    fnc[0] = (hp * VLd + hm * VRd) + ((hp * Smd) * gmL + (hm * Spd) * gmR);
-    fnc[1] = hp * (VLd * p1L + Smd * (double)tL1) + hm * (VRd * p1R + Spd * (double)tR1);
-    fnc[2] = hp * (VLd * p2L + Smd * (double)tL2) + hm * (VRd * p2R + Spd * (double)tR2);
-    }
-    float kL = wL[2] * wL[2] + wL[3] * wL[3], kR = wR[2] * wR[2] + wR[3] * wR[3];
-    if (DIM == 3) { kL += wL[4] * wL[4]; kR += wR[4] * wR[4]; }
-    cmax = fmaxf(cL + sqrtf(kL), cR + sqrtf(kR));
+    float kL = __fmaf_rn(wL[2], wL[2], wL[3] * wL[3]), kR = __fmaf_rn(wR[2], wR[2], wR[3] * wR[3]);
+    if (DIM == 3) { kL = __fmaf_rn(wL[4], wL[4], kL); kR = __fmaf_rn(wR[4], wR[4], kR); }
+    cmax = fmaxf(cL + sqrt_ftz(kL), cR + sqrt_ftz(kR));
 }
 
 // ------------------------------------------------------------------------------------------------
-// WENO5 face value, epsilon-free weights from smoothness ratios with a NaN guard.
-// side = +1: value at the right face of the centre cell c; side = -1: at its left face.
+// WENO5 face values (WENO5.H:12-75), epsilon-free weights from smoothness ratios with a NaN guard.
+// side = +1: value at the right face of the centre cell c; side = -1: at its left face. The two faces
+// of a cell share the indicators, the ratios and their squares, which are formed once for both (12
+// divisions for two face values; a face value formed alone takes 9), with the reference's operations.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ double weno5(double f_mm, double f_m, double f_c, double f_p, double f_pp, int side) {
-    double q0, q1, q2, d0, d2;
-    if (side == 1) {
-        q0 = (f_c + (2.0 / 3.0) * (f_p - f_c)) - (1.0 / 6.0) * (f_pp - f_p);
-        q1 = (f_c + (1.0 / 6.0) * (f_c - f_m)) + (1.0 / 3.0) * (f_p - f_c);
-        q2 = (f_c - (1.0 / 3.0) * (f_m - f_mm)) + (5.0 / 6.0) * (f_c - f_m);
-        d0 = 3.0 / 10.0;
-        d2 = 1.0 / 10.0;
-    } else {
-        q0 = (f_c - (5.0 / 6.0) * (f_p - f_c)) + (1.0 / 3.0) * (f_pp - f_p);
-        q1 = (f_c - (1.0 / 3.0) * (f_c - f_m)) - (1.0 / 6.0) * (f_p - f_c);
-        q2 = (f_c + (1.0 / 6.0) * (f_m - f_mm)) - (2.0 / 3.0) * (f_c - f_m);
-        d0 = 1.0 / 10.0;
-        d2 = 3.0 / 10.0;
-    }
-    const double d1 = (1.0 - d0) - d2;
-    const double a = f_p - f_c, b = f_pp - f_p, c = f_c - f_m, g = f_m - f_mm;
-    const double IS0 = ((10.0 / 3.0) * a) * a - ((11.0 / 3.0) * a) * b + ((4.0 / 3.0) * b) * b;
-    const double IS1 = (-(5.0 / 3.0) * c) * a + ((4.0 / 3.0) * c) * c + ((4.0 / 3.0) * a) * a;
-    const double IS2 = ((10.0 / 3.0) * c) * c - ((11.0 / 3.0) * g) * c + ((4.0 / 3.0) * g) * g;
-    double IS01 = IS0 / IS1;
-    if (isnan(IS01)) IS01 = 1.0;
-    const double IS10 = 1.0 / IS01;
-    double IS02 = IS0 / IS2;
-    if (isnan(IS02)) IS02 = 1.0;
-    const double IS20 = 1.0 / IS02;
-    double IS12 = IS1 / IS2;
-    if (isnan(IS12)) IS12 = 1.0;
-    const double IS21 = 1.0 / IS12;
-    const double w0 = d0 / ((d0 + (IS01 * IS01) * d1) + (IS02 * IS02) * d2);
-    const double w1 = d1 / (((IS10 * IS10) * d0 + d1) + (IS12 * IS12) * d2);
-    const double w2 = d2 / (((IS20 * IS20) * d0 + (IS21 * IS21) * d1) + d2);
-    double f = 0.0;
-    f += w0 * q0;
-    f += w1 * q1;
-    f += w2 * q2;
-    return f;
-}
-
-// WENO5 candidate values q and nonlinear weights w separately (WENO5.H:12-75), for the bounded
-// variant, which reconstructs the volume fractions with the weights of the partial densities.
-__device__ __forceinline__ void weno5_parts(double f_mm, double f_m, double f_c, double f_p, double f_pp, int side,
-                                            double q[3], double* w) {
-    double d0, d2;
+__device__ __forceinline__ void weno5_cand(double f_mm, double f_m, double f_c, double f_p, double f_pp, int side,
+                                           double q[3]) {
     if (side == 1) {
         q[0] = (f_c + (2.0 / 3.0) * (f_p - f_c)) - (1.0 / 6.0) * (f_pp - f_p);
         q[1] = (f_c + (1.0 / 6.0) * (f_c - f_m)) + (1.0 / 3.0) * (f_p - f_c);
         q[2] = (f_c - (1.0 / 3.0) * (f_m - f_mm)) + (5.0 / 6.0) * (f_c - f_m);
-        d0 = 3.0 / 10.0;
-        d2 = 1.0 / 10.0;
     } else {
         q[0] = (f_c - (5.0 / 6.0) * (f_p - f_c)) + (1.0 / 3.0) * (f_pp - f_p);
         q[1] = (f_c - (1.0 / 3.0) * (f_c - f_m)) - (1.0 / 6.0) * (f_p - f_c);
         q[2] = (f_c + (1.0 / 6.0) * (f_m - f_mm)) - (2.0 / 3.0) * (f_c - f_m);
-        d0 = 1.0 / 10.0;
-        d2 = 3.0 / 10.0;
     }
-    if (!w) return;
-    const double d1 = (1.0 - d0) - d2;
+}
+
+// FP64 quotients without the range handling of a division, for operands that the caller knows to be
+// positive and far from over- and underflow.
+// approx_rcp: within about one unit in the last place of 1/b, the hardware's 20-bit estimate refined by the
+// cubic step y (1 + e + e^2), e = 1 - b y. refine_rcp: the correctly rounded 1/b from a y within a few units
+// of it: a first step rounded upwards, so that the result is within one unit and not below where b's
+// significand is all ones, then P. Markstein's step y + y (1 - b y), whose residual is exact in an FMA
+// ("Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).
+// div_rn: the correctly rounded a/b from y = 1/b so rounded, by the same paper's q + (a - b q) y. One
+// reciprocal serves every quotient over the same denominator, and none of it branches.
+__device__ __forceinline__ double approx_rcp(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    return fma(fma(e, e, e), y, y);
+}
+__device__ __forceinline__ double refine_rcp(double b, double y) {
+    y = __fma_ru(fma(-b, y, 1.0), y, y);
+    return fma(fma(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ double rcp_rn(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = fma(-b, y, 1.0);
+    y = __fma_ru(fma(e, e, e), y, y);
+    e = fma(-b, y, 1.0);
+    return fma(e, y, y);
+}
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+// sqrt(x), x >= 0, within about one unit in the last place (mixed form): two Newton steps
+// y (3 - x y^2)/2 on the hardware's estimate of 1/sqrt(x), then x y with its residual folded in.
+__device__ __forceinline__ double approx_sqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = y * fma(-0.5 * x, y * y, 1.5);
+    const double s = x * y;
+    const double r = fma(fma(-s, s, x), 0.5 * y, s);
+    return (x > 0.0) ? r : x;
+}
+
+// Weights of the right face (wp) and the left face (wm) of the centre cell. Where the three indicators lie
+// within 2^+-240 (or all vanish, which the ratio form treats as all equal) the quotients are formed without
+// branches: three reciprocals serve the six ratios, and a face's first denominator, scaled by the squared
+// ratios, gives the reciprocals of the other two (exact relations, so only the last bits need correcting).
+// Other cells, at the edge of a uniform region above all, divide as the reference writes it. Both give
+// the correctly rounded quotients.
+__device__ __forceinline__ void weno5_weights(double f_mm, double f_m, double f_c, double f_p, double f_pp, double wp[3],
+                                              double wm[3]) {
     const double a = f_p - f_c, b = f_pp - f_p, c = f_c - f_m, g = f_m - f_mm;
-    const double IS0 = ((10.0 / 3.0) * a) * a - ((11.0 / 3.0) * a) * b + ((4.0 / 3.0) * b) * b;
-    const double IS1 = (-(5.0 / 3.0) * c) * a + ((4.0 / 3.0) * c) * c + ((4.0 / 3.0) * a) * a;
-    const double IS2 = ((10.0 / 3.0) * c) * c - ((11.0 / 3.0) * g) * c + ((4.0 / 3.0) * g) * g;
+    double IS0 = ((10.0 / 3.0) * a) * a - ((11.0 / 3.0) * a) * b + ((4.0 / 3.0) * b) * b;
+    double IS1 = (-(5.0 / 3.0) * c) * a + ((4.0 / 3.0) * c) * c + ((4.0 / 3.0) * a) * a;
+    double IS2 = ((10.0 / 3.0) * c) * c - ((11.0 / 3.0) * g) * c + ((4.0 / 3.0) * g) * g;
+    if (IS0 == 0.0 && IS1 == 0.0 && IS2 == 0.0) IS0 = IS1 = IS2 = 1.0;
+    const unsigned h0 = (unsigned)__double2hiint(IS0), h1 = (unsigned)__double2hiint(IS1),
+                   h2 = (unsigned)__double2hiint(IS2);
+    constexpr unsigned LO = (1023u - 240u) << 20, HI = (1023u + 240u) << 20;
+    if (min(min(h0, h1), h2) >= LO && max(max(h0, h1), h2) < HI) {
+        const double y0 = approx_rcp(IS0), y1 = rcp_rn(IS1), y2 = rcp_rn(IS2);
+        const double IS01 = div_rn(IS0, IS1, y1), IS02 = div_rn(IS0, IS2, y2), IS12 = div_rn(IS1, IS2, y2);
+        // 1/IS01 from its close approximation IS1/IS0, and so on
+        const double IS10 = refine_rcp(IS01, IS1 * y0), IS20 = refine_rcp(IS02, IS2 * y0), IS21 = refine_rcp(IS12, IS2 * y1);
+        const double s01 = IS01 * IS01, s02 = IS02 * IS02, s10 = IS10 * IS10, s12 = IS12 * IS12, s20 = IS20 * IS20,
+                     s21 = IS21 * IS21;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double d0 = k ? 1.0 / 10.0 : 3.0 / 10.0, d2 = k ? 3.0 / 10.0 : 1.0 / 10.0;
+            const double d1 = (1.0 - d0) - d2;
+            double* w = k ? wm : wp;
+            const double D0 = (d0 + s01 * d1) + s02 * d2, D1 = (s10 * d0 + d1) + s12 * d2, D2 = (s20 * d0 + s21 * d1) + d2;
+            const double r0 = rcp_rn(D0), r1 = refine_rcp(D1, r0 * s01), r2 = refine_rcp(D2, r0 * s02);
+            w[0] = div_rn(d0, D0, r0);
+            w[1] = div_rn(d1, D1, r1);
+            w[2] = div_rn(d2, D2, r2);
+        }
+        return;
+    }
     double IS01 = IS0 / IS1;
     if (isnan(IS01)) IS01 = 1.0;
-    const double IS10 = 1.0 / IS01;
     double IS02 = IS0 / IS2;
     if (isnan(IS02)) IS02 = 1.0;
-    const double IS20 = 1.0 / IS02;
     double IS12 = IS1 / IS2;
     if (isnan(IS12)) IS12 = 1.0;
-    const double IS21 = 1.0 / IS12;
-    w[0] = d0 / ((d0 + (IS01 * IS01) * d1) + (IS02 * IS02) * d2);
-    w[1] = d1 / (((IS10 * IS10) * d0 + d1) + (IS12 * IS12) * d2);
-    w[2] = d2 / (((IS20 * IS20) * d0 + (IS21 * IS21) * d1) + d2);
+    const double IS10 = 1.0 / IS01, IS20 = 1.0 / IS02, IS21 = 1.0 / IS12;
+    const double s01 = IS01 * IS01, s02 = IS02 * IS02, s10 = IS10 * IS10, s12 = IS12 * IS12, s20 = IS20 * IS20,
+                 s21 = IS21 * IS21;
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+        const double d0 = k ? 1.0 / 10.0 : 3.0 / 10.0, d2 = k ? 3.0 / 10.0 : 1.0 / 10.0;
+        const double d1 = (1.0 - d0) - d2;
+        const double w0 = d0 / ((d0 + s01 * d1) + s02 * d2);
+        const double w1 = d1 / ((s10 * d0 + d1) + s12 * d2);
+        const double w2 = d2 / ((s20 * d0 + s21 * d1) + d2);
+        if (k == 0) {
+            wp[0] = w0;
+            wp[1] = w1;
+            wp[2] = w2;
+        } else {
+            wm[0] = w0;
+            wm[1] = w1;
+            wm[2] = w2;
+        }
+    }
 }
 
 __device__ __forceinline__ double weno_sum(const double q[3], const double w[3]) {
@@ -847,6 +908,23 @@ __device__ __forceinline__ double weno_sum(const double q[3], const double w[3])
     f += w[1] * q[1];
     f += w[2] * q[2];
     return f;
+}
+
+// Both face values of the centre cell: vp at its right face, vm at its left face.
+__device__ __forceinline__ void weno5_both(double f_mm, double f_m, double f_c, double f_p, double f_pp, double& vp,
+                                           double& vm) {
+    double wp[3], wm[3], q[3];
+    weno5_weights(f_mm, f_m, f_c, f_p, f_pp, wp, wm);
+    weno5_cand(f_mm, f_m, f_c, f_p, f_pp, 1, q);
+    vp = weno_sum(q, wp);
+    weno5_cand(f_mm, f_m, f_c, f_p, f_pp, -1, q);
+    vm = weno_sum(q, wm);
+}
+
+__device__ __forceinline__ double weno5(double f_mm, double f_m, double f_c, double f_p, double f_pp, int side) {
+    double vp, vm;
+    weno5_both(f_mm, f_m, f_c, f_p, f_pp, vp, vm);
+    return (side == 1) ? vp : vm;
 }
 
 // Positivity limiter of a cell with face values fL (right face) and fR (left face), lower bound 0
@@ -859,6 +937,22 @@ __device__ __forceinline__ double bound_min_theta(double f_c, double fL, double 
     if (fR < mn) mn = fR;
     const double th = dmax(0.0, f_c - 0.0) / dmax(0.0, f_c - mn);
     return dmin(1.0, th);
+}
+
+// WENO5 face values (L right face, R left face) of a mass fr and a volume fraction fa, both with the
+// weights of the mass.
+__device__ __forceinline__ void bounded_cell5(const double* fr, const double* fa, double& rL, double& rR, double& aL,
+                                              double& aR) {
+    double q[3], wp[3], wm[3];
+    weno5_weights(fr[0], fr[1], fr[2], fr[3], fr[4], wp, wm);
+    weno5_cand(fr[0], fr[1], fr[2], fr[3], fr[4], 1, q);
+    rL = weno_sum(q, wp);
+    weno5_cand(fa[0], fa[1], fa[2], fa[3], fa[4], 1, q);
+    aL = weno_sum(q, wp);
+    weno5_cand(fr[0], fr[1], fr[2], fr[3], fr[4], -1, q);
+    rR = weno_sum(q, wm);
+    weno5_cand(fa[0], fa[1], fa[2], fa[3], fa[4], -1, q);
+    aR = weno_sum(q, wm);
 }
 
 // Bounded WENO5 (WENO5B) face values of the masses and volume fractions of one cell (stencil values
@@ -882,15 +976,7 @@ __device__ __forceinline__ void weno5b_masses_both(const double* ar1, const doub
 #pragma unroll
         for (int s = 0; s < 5; ++s) fa[s] = (k == 0) ? al1[s] : 1.0 - al1[s];
         ac[k] = fa[2];
-        double q[3], w[3], qa[3];
-        weno5_parts(fr[0], fr[1], fr[2], fr[3], fr[4], 1, q, w);
-        rL[k] = weno_sum(q, w);
-        weno5_parts(fa[0], fa[1], fa[2], fa[3], fa[4], 1, qa, nullptr);
-        aL[k] = weno_sum(qa, w);
-        weno5_parts(fr[0], fr[1], fr[2], fr[3], fr[4], -1, q, w);
-        rR[k] = weno_sum(q, w);
-        weno5_parts(fa[0], fa[1], fa[2], fa[3], fa[4], -1, qa, nullptr);
-        aR[k] = weno_sum(qa, w);
+        bounded_cell5(fr, fa, rL[k], rR[k], aL[k], aR[k]);
         const double th_r = bound_min_theta(fr[2], rL[k], rR[k], W);
         const double th_a = bound_min_theta(fa[2], aL[k], aR[k], W);
         const double th = dmin(th_r, th_a);
@@ -940,53 +1026,72 @@ __device__ __forceinline__ void weno5b_masses(const double* ar1, const double* a
 // rounding of the weights, and the FP32 error scales with the correction, not with |f|. The
 // weights are the reference's ratio-form weights (include/Operators_FV/WENO5.H:44-75) rewritten
 // with one reciprocal: with r01 = IS0/IS1 and r02 = IS0/IS2, D = d0 + r01^2 d1 + r02^2 d2 and
-// w0 = d0/D, w1 = d1 r01^2/D, w2 = d2 r02^2/D (the same weights in exact arithmetic); where a
-// smoothness indicator vanishes or a ratio is huge, the ratio form with its NaN guard is used.
+// w0 = d0/D, w1 = d1 r01^2/D, w2 = d2 r02^2/D (the same weights in exact arithmetic). The two faces
+// of a cell share the indicators and the ratios; only d0 and d2 change places. Every operation is
+// written out (no contraction), so a value that is computed once for both faces, or carried from
+// cell to cell of a line, has the bits it has when it is computed for one face alone.
+//
+// Indicators: three times the reference's (integer coefficients; only ratios enter), each a positive
+// definite form of two differences (smallest eigenvalue 0.73), so rounding cannot make one negative.
+// kWenoFloor, far below the square of any FP32 difference of a resolved field, stands in for zero: all
+// indicators zero gives the linear weights, some zero gives those stencils their share of them, as the
+// reference's NaN guard does. Ratios are clamped at 1e18, where the weights are 0 or 1 to FP32
+// precision, so that the squares stay finite.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void weno5_f32_parts(float f_mm, float f_m, float f_c, float f_p, float f_pp, int side,
-                                                float e[3], float* w) {
-    const float a = f_p - f_c, b = f_pp - f_p, c = f_c - f_m, g = f_m - f_mm;
-    float d0, d2;
+constexpr float kWenoFloor = 1.0e-36f;
+
+// r01^2 and r02^2 from the undivided differences g, c, a, b of the five cells.
+__device__ __forceinline__ void weno5_ratios_f32(float g, float c, float a, float b, float& s01, float& s02) {
+    const float IS0 = __fmaf_rn(10.0f, a * a, __fmaf_rn(-11.0f, a * b, __fmaf_rn(4.0f, b * b, kWenoFloor)));
+    const float IS1 = __fmaf_rn(-5.0f, c * a, __fmaf_rn(4.0f, c * c, __fmaf_rn(4.0f, a * a, kWenoFloor)));
+    const float IS2 = __fmaf_rn(10.0f, c * c, __fmaf_rn(-11.0f, g * c, __fmaf_rn(4.0f, g * g, kWenoFloor)));
+    const float r01 = fminf(IS0 * rcp_ftz(IS1), 1.0e18f);
+    const float r02 = fminf(IS0 * rcp_ftz(IS2), 1.0e18f);
+    s01 = r01 * r01;
+    s02 = r02 * r02;
+}
+
+// Weights of the right face (side +1: d = 0.3, 0.6, 0.1) or the left face (d = 0.1, 0.6, 0.3).
+__device__ __forceinline__ void weno5_weights_f32(float s01, float s02, int side, float* w) {
+    const float d0 = (side == 1) ? 3.0f : 1.0f, d2 = (side == 1) ? 1.0f : 3.0f;
+    const float x1 = 6.0f * s01, x2 = d2 * s02;
+    const float inv = rcp_ftz(d0 + x1 + x2);
+    w[0] = d0 * inv;
+    w[1] = x1 * inv;
+    w[2] = x2 * inv;
+}
+
+// sum_k w_k (q_k - f_c) of one face.
+__device__ __forceinline__ float weno5_corr_f32(float g, float c, float a, float b, int side, const float* w) {
+    float e0, e1, e2;  // 6 (q_k - f_c)
     if (side == 1) {
-        e[0] = __fmaf_rn(2.0f / 3.0f, a, -(1.0f / 6.0f) * b);
-        e[1] = __fmaf_rn(1.0f / 6.0f, c, (1.0f / 3.0f) * a);
-        e[2] = __fmaf_rn(-(1.0f / 3.0f), g, (5.0f / 6.0f) * c);
-        d0 = 0.3f;
-        d2 = 0.1f;
+        e0 = __fmaf_rn(4.0f, a, -b);
+        e1 = __fmaf_rn(2.0f, a, c);
+        e2 = __fmaf_rn(5.0f, c, -2.0f * g);
     } else {
-        e[0] = __fmaf_rn(-(5.0f / 6.0f), a, (1.0f / 3.0f) * b);
-        e[1] = __fmaf_rn(-(1.0f / 3.0f), c, -(1.0f / 6.0f) * a);
-        e[2] = __fmaf_rn(1.0f / 6.0f, g, -(2.0f / 3.0f) * c);
-        d0 = 0.1f;
-        d2 = 0.3f;
+        e0 = __fmaf_rn(-5.0f, a, 2.0f * b);
+        e1 = -__fmaf_rn(2.0f, c, a);
+        e2 = __fmaf_rn(-4.0f, c, g);
     }
-    if (!w) return;
-    const float d1 = 0.6f;
-    const float IS0 = __fmaf_rn((10.0f / 3.0f) * a, a, __fmaf_rn(-(11.0f / 3.0f) * a, b, (4.0f / 3.0f) * b * b));
-    const float IS1 = __fmaf_rn(-(5.0f / 3.0f) * c, a, (4.0f / 3.0f) * __fmaf_rn(c, c, a * a));
-    const float IS2 = __fmaf_rn((10.0f / 3.0f) * c, c, __fmaf_rn(-(11.0f / 3.0f) * g, c, (4.0f / 3.0f) * g * g));
-    // Where some indicators vanish the ratio form gives the stencils with IS = 0 the weight in
-    // proportion to their linear weights and the others none (a uniform stencil: d_k); otherwise the
-    // one-reciprocal form, with the ratios clamped at 1e18 where the weights are 0 or 1 to FP32
-    // precision anyway. Both are evaluated without branches.
-    const bool z0 = (IS0 == 0.0f), z1 = (IS1 == 0.0f), z2 = (IS2 == 0.0f);
-    const bool anyz = z0 | z1 | z2;
-    const float szero = (z0 ? d0 : 0.0f) + (z1 ? d1 : 0.0f) + (z2 ? d2 : 0.0f);
-    // |ratio|: an indicator can round slightly below zero; the clamp then also bounds the square
-    const float r01 = fminf(fabsf(IS0 * __fdividef(1.0f, IS1)), 1.0e18f);
-    const float r02 = fminf(fabsf(IS0 * __fdividef(1.0f, IS2)), 1.0e18f);
-    const float s01 = anyz ? 0.0f : r01 * r01, s02 = anyz ? 0.0f : r02 * r02;
-    const float den = anyz ? szero : __fmaf_rn(s01, d1, __fmaf_rn(s02, d2, d0));
-    const float inv = __fdividef(1.0f, den);
-    w[0] = (anyz ? (z0 ? d0 : 0.0f) : d0) * inv;
-    w[1] = (anyz ? (z1 ? d1 : 0.0f) : d1 * s01) * inv;
-    w[2] = (anyz ? (z2 ? d2 : 0.0f) : d2 * s02) * inv;
+    return __fmaf_rn(w[0], e0, __fmaf_rn(w[1], e1, w[2] * e2)) * (1.0f / 6.0f);
+}
+
+// Both face values of the centre cell: vp at its right face, vm at its left face.
+__device__ __forceinline__ void weno5_both_f32(float f_mm, float f_m, float f_c, float f_p, float f_pp, float& vp,
+                                               float& vm) {
+    const float a = f_p - f_c, b = f_pp - f_p, c = f_c - f_m, g = f_m - f_mm;
+    float s01, s02, wp[3], wm[3];
+    weno5_ratios_f32(g, c, a, b, s01, s02);
+    weno5_weights_f32(s01, s02, 1, wp);
+    weno5_weights_f32(s01, s02, -1, wm);
+    vp = f_c + weno5_corr_f32(g, c, a, b, 1, wp);
+    vm = f_c + weno5_corr_f32(g, c, a, b, -1, wm);
 }
 
 __device__ __forceinline__ float weno5_f32(float f_mm, float f_m, float f_c, float f_p, float f_pp, int side) {
-    float e[3], w[3];
-    weno5_f32_parts(f_mm, f_m, f_c, f_p, f_pp, side, e, w);
-    return f_c + __fmaf_rn(w[0], e[0], __fmaf_rn(w[1], e[1], w[2] * e[2]));
+    float vp, vm;
+    weno5_both_f32(f_mm, f_m, f_c, f_p, f_pp, vp, vm);
+    return (side == 1) ? vp : vm;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1121,9 +1226,25 @@ __device__ __forceinline__ float bound_min_theta_f32(float f_c, float fL, float 
     return fminf(1.0f, __fdividef(fmaxf(0.0f, f_c), den));
 }
 
-// WENO5B masses and volume fraction in FP32 (same steps as weno5b_masses).
-__device__ __forceinline__ void weno5b_masses_f32(const float* ar1, const float* ar2, const float* al1, int side,
-                                                  float& a1r1_f, float& a2r2_f, float& alpha1_f) {
+// The FP32 counterpart of bounded_cell5.
+__device__ __forceinline__ void bounded_cell5_f32(const float* fr, const float* fa, float& rL, float& rR, float& aL,
+                                                  float& aR) {
+    const float g = fr[1] - fr[0], c = fr[2] - fr[1], a = fr[3] - fr[2], b = fr[4] - fr[3];
+    const float ga = fa[1] - fa[0], ca = fa[2] - fa[1], aa = fa[3] - fa[2], ba = fa[4] - fa[3];
+    float s01, s02, wp[3], wm[3];
+    weno5_ratios_f32(g, c, a, b, s01, s02);
+    weno5_weights_f32(s01, s02, 1, wp);
+    weno5_weights_f32(s01, s02, -1, wm);
+    rL = fr[2] + weno5_corr_f32(g, c, a, b, 1, wp);
+    aL = fa[2] + weno5_corr_f32(ga, ca, aa, ba, 1, wp);
+    rR = fr[2] + weno5_corr_f32(g, c, a, b, -1, wm);
+    aR = fa[2] + weno5_corr_f32(ga, ca, aa, ba, -1, wm);
+}
+
+// WENO5B masses and volume fraction in FP32 (same steps as weno5b_masses_both): the right-face values to
+// Wp[0..2] (a1r1, a2r2, alpha1), the left-face values to Wm[0..2].
+__device__ __forceinline__ void weno5b_masses_both_f32(const float* ar1, const float* ar2, const float* al1, float* Wp,
+                                                       float* Wm) {
     float rL[2], rR[2], aL[2], aR[2], ac[2];
     float sumL = 0.0f, sumR = 0.0f;
 #pragma unroll
@@ -1133,15 +1254,7 @@ __device__ __forceinline__ void weno5b_masses_f32(const float* ar1, const float*
 #pragma unroll
         for (int s = 0; s < 5; ++s) fa[s] = (k == 0) ? al1[s] : 1.0f - al1[s];
         ac[k] = fa[2];
-        float e[3], w[3], ea[3];
-        weno5_f32_parts(fr[0], fr[1], fr[2], fr[3], fr[4], 1, e, w);
-        weno5_f32_parts(fa[0], fa[1], fa[2], fa[3], fa[4], 1, ea, nullptr);
-        rL[k] = fr[2] + __fmaf_rn(w[0], e[0], __fmaf_rn(w[1], e[1], w[2] * e[2]));
-        aL[k] = fa[2] + __fmaf_rn(w[0], ea[0], __fmaf_rn(w[1], ea[1], w[2] * ea[2]));
-        weno5_f32_parts(fr[0], fr[1], fr[2], fr[3], fr[4], -1, e, w);
-        weno5_f32_parts(fa[0], fa[1], fa[2], fa[3], fa[4], -1, ea, nullptr);
-        rR[k] = fr[2] + __fmaf_rn(w[0], e[0], __fmaf_rn(w[1], e[1], w[2] * e[2]));
-        aR[k] = fa[2] + __fmaf_rn(w[0], ea[0], __fmaf_rn(w[1], ea[1], w[2] * ea[2]));
+        bounded_cell5_f32(fr, fa, rL[k], rR[k], aL[k], aR[k]);
         const float th = fminf(bound_min_theta_f32(fr[2], rL[k], rR[k]), bound_min_theta_f32(fa[2], aL[k], aR[k]));
         rL[k] = __fmaf_rn(th, rL[k] - fr[2], fr[2]);
         aL[k] = __fmaf_rn(th, aL[k] - fa[2], fa[2]);
@@ -1161,12 +1274,22 @@ __device__ __forceinline__ void weno5b_masses_f32(const float* ar1, const float*
         aR[k] *= iR;
         Th = fminf(Th, fminf(bound_min_theta_f32(rc, rL[k], rR[k]), bound_min_theta_f32(ac[k], aL[k], aR[k])));
     }
-    const float r1 = (side == 1) ? rL[0] : rR[0];
-    const float r2 = (side == 1) ? rL[1] : rR[1];
-    const float a1 = (side == 1) ? aL[0] : aR[0];
-    a1r1_f = __fmaf_rn(Th, r1 - ar1[2], ar1[2]);
-    a2r2_f = __fmaf_rn(Th, r2 - ar2[2], ar2[2]);
-    alpha1_f = __fmaf_rn(Th, a1 - al1[2], al1[2]);
+    Wp[0] = __fmaf_rn(Th, rL[0] - ar1[2], ar1[2]);
+    Wp[1] = __fmaf_rn(Th, rL[1] - ar2[2], ar2[2]);
+    Wp[2] = __fmaf_rn(Th, aL[0] - al1[2], al1[2]);
+    Wm[0] = __fmaf_rn(Th, rR[0] - ar1[2], ar1[2]);
+    Wm[1] = __fmaf_rn(Th, rR[1] - ar2[2], ar2[2]);
+    Wm[2] = __fmaf_rn(Th, aR[0] - al1[2], al1[2]);
+}
+
+__device__ __forceinline__ void weno5b_masses_f32(const float* ar1, const float* ar2, const float* al1, int side,
+                                                  float& a1r1_f, float& a2r2_f, float& alpha1_f) {
+    float Wp[3], Wm[3];
+    weno5b_masses_both_f32(ar1, ar2, al1, Wp, Wm);
+    const float* Wf = (side == 1) ? Wp : Wm;
+    a1r1_f = Wf[0];
+    a2r2_f = Wf[1];
+    alpha1_f = Wf[2];
 }
 
 // Bounded WENO face values of NP phases. WENO5B, ORDER 5:
@@ -1174,13 +1297,14 @@ __device__ __forceinline__ void weno5b_masses_f32(const float* ar1, const float*
 // WENO3B, ORDER 3: include/Operators_Compressible5Eq/FVM_Reconstruction2Face_Conservative_WENO3B_D_Compressible5Eq.H:95-236,
 // the six-equation and N-phase counterparts (same steps). Per phase: the WENO faces of alpha_k rho_k and of
 // alpha_k (with the weights of alpha_k rho_k), one positivity theta for both; the faces divided by sum alpha_k;
-// one common theta over all phases applied to the face of side `side`. r(k, s) and a(k, s) give alpha_k rho_k
-// and alpha_k of stencil cell s = 0..ORDER-1 (centre ORDER/2); the results go to rf[k], af[k]. PT = double:
+// one common theta over all phases. r(k, s) and a(k, s) give alpha_k rho_k
+// and alpha_k of stencil cell s = 0..ORDER-1 (centre ORDER/2); the right-face values go to rp[k], ap[k], the
+// left-face values to rm[k], am[k]. PT = double:
 // the reference's arithmetic (quadrature weight 1/12 for ORDER 5, 1/6 for ORDER 3); PT = float: the mixed form.
 // Wq > 0 replaces the quadrature weight (the bound-preserving path runs the fifth-order stencil with
 // weight 1/6 for WENO3 / WENO3B, FiniteVolume_Parameter.H:114-127).
 template <int NP, int ORDER, class PT, class FR, class FA>
-__device__ __forceinline__ void bounded_phases(FR r, FA a, int side, PT* rf, PT* af, double Wq = 0.0) {
+__device__ __forceinline__ void bounded_phases_both(FR r, FA a, PT* rp, PT* ap, PT* rm, PT* am, double Wq = 0.0) {
     constexpr bool F32 = std::is_same<PT, float>::value;
     constexpr int C = ORDER / 2;
     const double W = (Wq > 0.0) ? Wq : ((ORDER == 5) ? 1.0 / 12.0 : 1.0 / 6.0);
@@ -1214,25 +1338,9 @@ __device__ __forceinline__ void bounded_phases(FR r, FA a, int side, PT* rf, PT*
             weno3_qw(fa[0], fa[1], fa[2], -1, qa, wa);
             aR[k] = weno3_sum(qa, w);
         } else if constexpr (F32) {
-            float e[3], w[3], ea[3];
-            weno5_f32_parts(fr[0], fr[1], fr[2], fr[3], fr[4], 1, e, w);
-            weno5_f32_parts(fa[0], fa[1], fa[2], fa[3], fa[4], 1, ea, nullptr);
-            rL[k] = fr[2] + __fmaf_rn(w[0], e[0], __fmaf_rn(w[1], e[1], w[2] * e[2]));
-            aL[k] = fa[2] + __fmaf_rn(w[0], ea[0], __fmaf_rn(w[1], ea[1], w[2] * ea[2]));
-            weno5_f32_parts(fr[0], fr[1], fr[2], fr[3], fr[4], -1, e, w);
-            weno5_f32_parts(fa[0], fa[1], fa[2], fa[3], fa[4], -1, ea, nullptr);
-            rR[k] = fr[2] + __fmaf_rn(w[0], e[0], __fmaf_rn(w[1], e[1], w[2] * e[2]));
-            aR[k] = fa[2] + __fmaf_rn(w[0], ea[0], __fmaf_rn(w[1], ea[1], w[2] * ea[2]));
+            bounded_cell5_f32(fr, fa, rL[k], rR[k], aL[k], aR[k]);
         } else {
-            double q[3], w[3], qa[3];
-            weno5_parts(fr[0], fr[1], fr[2], fr[3], fr[4], 1, q, w);
-            rL[k] = weno_sum(q, w);
-            weno5_parts(fa[0], fa[1], fa[2], fa[3], fa[4], 1, qa, nullptr);
-            aL[k] = weno_sum(qa, w);
-            weno5_parts(fr[0], fr[1], fr[2], fr[3], fr[4], -1, q, w);
-            rR[k] = weno_sum(q, w);
-            weno5_parts(fa[0], fa[1], fa[2], fa[3], fa[4], -1, qa, nullptr);
-            aR[k] = weno_sum(qa, w);
+            bounded_cell5(fr, fa, rL[k], rR[k], aL[k], aR[k]);
         }
         if constexpr (F32) {
             th = fminf(bound_min_theta_f32(fr[C], rL[k], rR[k], (float)W),
@@ -1270,14 +1378,30 @@ __device__ __forceinline__ void bounded_phases(FR r, FA a, int side, PT* rf, PT*
     }
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
-        const PT rs = (side == 1) ? rL[k] : rR[k], as = (side == 1) ? aL[k] : aR[k];
+        const PT rc = r(k, C), ac = a(k, C);
         if constexpr (F32) {
-            rf[k] = __fmaf_rn(Th, rs - r(k, C), r(k, C));
-            af[k] = __fmaf_rn(Th, as - a(k, C), a(k, C));
+            rp[k] = __fmaf_rn(Th, rL[k] - rc, rc);
+            ap[k] = __fmaf_rn(Th, aL[k] - ac, ac);
+            rm[k] = __fmaf_rn(Th, rR[k] - rc, rc);
+            am[k] = __fmaf_rn(Th, aR[k] - ac, ac);
         } else {
-            rf[k] = r(k, C) + Th * (rs - r(k, C));
-            af[k] = a(k, C) + Th * (as - a(k, C));
+            rp[k] = rc + Th * (rL[k] - rc);
+            ap[k] = ac + Th * (aL[k] - ac);
+            rm[k] = rc + Th * (rR[k] - rc);
+            am[k] = ac + Th * (aR[k] - ac);
         }
+    }
+}
+
+// The face `side` (+1 right, -1 left) alone.
+template <int NP, int ORDER, class PT, class FR, class FA>
+__device__ __forceinline__ void bounded_phases(FR r, FA a, int side, PT* rf, PT* af, double Wq = 0.0) {
+    PT rp[NP], ap[NP], rm[NP], am[NP];
+    bounded_phases_both<NP, ORDER, PT>(r, a, rp, ap, rm, am, Wq);
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        rf[k] = (side == 1) ? rp[k] : rm[k];
+        af[k] = (side == 1) ? ap[k] : am[k];
     }
 }
 

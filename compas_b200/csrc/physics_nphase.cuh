@@ -193,9 +193,6 @@ struct FiveEqN {
         double WL[N], WR[N];
         cons2prim(WL, UL, e, err);
         cons2prim(WR, UR, e, err);
-        double FL[N], FR[N];
-        flux(FL, UL, WL, d);
-        flux(FR, UR, WR, d);
         const double cL = sound_speed(WL, e, id_k, err);
         const double cR = sound_speed(WR, e, id_k, err);
         const double VL = pick<D>(WL + IM, d), VR = pick<D>(WR + IM, d);
@@ -214,25 +211,39 @@ struct FiveEqN {
         }
         const double S_Star = (((pR - pL) + (rhoL * VL) * (SL - VL)) - (rhoR * VR) * (SR - VR)) /
                               (rhoL * (SL - VL) - rhoR * (SR - VR));
-        const double s = sgn0(S_Star);
-        const double hp = 0.5 * (1.0 + s), hm = 0.5 * (1.0 - s);
-        const double fL = (SL - VL) / (SL - S_Star);
-        const double fR = (SR - VR) / (SR - S_Star);
-        double vel = hp * VL + hm * VR;
-        vel = vel + ((hp * Sm) * (fL - 1.0) + (hm * Sp) * (fR - 1.0));
-        fnc[0] = vel;
+        // the upwind side's star state, and both where S* is 0 (FiveEq::hllc_uw)
+        const bool left = S_Star > 0.0, both = !(left || S_Star < 0.0);
+        auto side = [&](bool lt, double* F, double& vel, double& dvel) {
+            const double V = lt ? VL : VR, p = lt ? pL : pR, rho = lt ? rhoL : rhoR, SK = lt ? SL : SR;
+            const double Sb = lt ? Sm : Sp;
+            double U[N], W[N];
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            double sL = fL * UL[i];
-            double sR = fR * UR[i];
-            if (i == IM + d) {
-                sL = sL + (fL * rhoL) * (S_Star - VL);
-                sR = sR + (fR * rhoR) * (S_Star - VR);
-            } else if (i == IE) {
-                sL = sL + (fL * (S_Star - VL)) * (rhoL * S_Star + pL / (SL - VL));
-                sR = sR + (fR * (S_Star - VR)) * (rhoR * S_Star + pR / (SR - VR));
+            for (int i = 0; i < N; ++i) {
+                U[i] = lt ? UL[i] : UR[i];
+                W[i] = lt ? WL[i] : WR[i];
             }
-            Fout[i] = hp * (FL[i] + Sm * (sL - UL[i])) + hm * (FR[i] + Sp * (sR - UR[i]));
+            flux(F, U, W, d);
+            const double f = (SK - V) / (SK - S_Star);
+            vel = V;
+            dvel = f - 1.0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                double star = f * U[i];
+                if (i == IM + d) star = star + (f * rho) * (S_Star - V);
+                else if (i == IE) star = star + (f * (S_Star - V)) * (rho * S_Star + p / (SK - V));
+                F[i] = F[i] + Sb * (star - U[i]);
+            }
+        };
+        double v, dv;
+        side(left || both, Fout, v, dv);
+        if (both) {
+            double F[N], vr, dvr;
+            side(false, F, vr, dvr);
+#pragma unroll
+            for (int i = 0; i < N; ++i) Fout[i] = 0.5 * Fout[i] + 0.5 * F[i];
+            fnc[0] = (0.5 * v + 0.5 * vr) + ((0.5 * Sm) * dv + (0.5 * Sp) * dvr);
+        } else {
+            fnc[0] = v + (left ? Sm : Sp) * dv;
         }
         const double qL = cL + sqrt(ksum<D>(WL + IM));
         const double qR = cR + sqrt(ksum<D>(WR + IM));
@@ -301,5 +312,165 @@ struct FiveEqN {
         prim2cons(Uf, Wf, e, err);
     }
 };
+
+// ---- mixed form ------------------------------------------------------------------------------------------
+// The consistent limiter on FP32 face primitives w, into FP64 (FiveEqN::consistent_limit without the
+// conversions to the conserved state and back, and with sd theta slope dx written theta (w - Wc); stiffened
+// gases). The two clamped ratios of Limiter_Consistent are each other's reciprocals: the one with the
+// larger denominator is formed, the other is then 0 or 1.
+template <class M, class PT>
+__device__ __forceinline__ void nphase_limit_mixed(double* W, const float* w, const PT* Wc, int wstr, double iden) {
+    constexpr int NP = M::NP;
+    const double ep = 1.0e-10;
+#pragma unroll
+    for (int n = 0; n < M::N; ++n) W[n] = w[n];
+    double da[NP], smax = 0.0, sum = 0.0;
+    int imax = 0;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        da[k] = W[M::IA + k] - (double)Wc[(M::IA + k) * wstr];
+        const double s = da[k] * iden;
+        sum += s;
+        if (k == 0 || fabs(smax) < fabs(s)) {
+            smax = s;
+            imax = k;
+        }
+    }
+    double t_max = 1.0, t_other = 1.0;
+    if (!(fabs(smax) < ep || fabs(sum) < ep)) {
+        const double rest = smax - sum;
+        const bool rl = fabs(rest) >= fabs(smax);
+        const double big = rl ? rest : smax, small = rl ? smax : rest;
+        const double q = dmax(small * approx_rcp(big), 0.0);
+        const double unit = (small * big > 0.0 || (small == 0.0 && big > 0.0)) ? 1.0 : 0.0;
+        t_other = rl ? q : unit;
+        t_max = rl ? unit : q;
+    }
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        const double th = (k == imax) ? t_max : t_other;
+        const double rc = Wc[k * wstr], ac = Wc[(M::IA + k) * wstr];
+        W[k] = fma(th, W[k] - rc, rc);
+        W[M::IA + k] = fma(th, da[k], ac);
+    }
+}
+
+template <class M>
+__device__ __forceinline__ double nphase_c_mixed(const double* W, double rho, const Eos& e, int id_k) {
+    const double p = W[M::IE];
+    double num = 0.0, den = 0.0;
+    if (id_k == 0) {
+#pragma unroll
+        for (int k = 0; k < M::NP; ++k) {
+            num = fma(W[M::IA + k], fma(e.Ak[k] + 1.0, p, e.Bk[k]), num);
+            den = fma(W[M::IA + k], e.Ak[k], den);
+        }
+        return approx_sqrt(num * approx_rcp(den * rho));
+    }
+#pragma unroll
+    for (int k = 0; k < M::NP; ++k)
+        den = fma(W[M::IA + k] * e.Ak[k], approx_rcp(fma(e.Ak[k] + 1.0, p, e.Bk[k])), den);
+    return approx_sqrt(approx_rcp(den * rho));
+}
+
+// HLLC of the N-phase model from FP64 face primitives (Riemann_HLLC_Compressible5Eq_NPhase.H; stiffened
+// gases): the star state of the upwind side only (both where S* is exactly 0), one reciprocal per
+// denominator.
+template <class M>
+__device__ __forceinline__ void nphase_hllc_mixed(double* Fout, double* fnc, double& cmax, const double* WL,
+                                                  const double* WR, const Eos& e, int d, int id_k) {
+    constexpr int N = M::N, D = M::D, NP = M::NP, IM = M::IM, IE = M::IE, IA = M::IA;
+    double rhoL = 0.0, rhoR = 0.0;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        rhoL += WL[k];
+        rhoR += WR[k];
+    }
+    const double cL = nphase_c_mixed<M>(WL, rhoL, e, id_k), cR = nphase_c_mixed<M>(WR, rhoR, e, id_k);
+    const double VL = pick<D>(WL + IM, d), VR = pick<D>(WR + IM, d);
+    const double Va = 0.5 * (VL + VR), ca = 0.5 * (cL + cR);
+    const double SL = dmin(Va - ca, VL - cL), SR = dmax(Va + ca, VR + cR);
+    const double mL = rhoL * (SL - VL), mR = rhoR * (SR - VR);
+    const double S = fma(mL, VL, (WR[IE] - WL[IE]) - mR * VR) * approx_rcp(mL - mR);
+    const double kL = ksum<D>(WL + IM), kR = ksum<D>(WR + IM);
+    auto side = [&](bool lt, double* F, double& vel) {
+        double W[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) W[n] = lt ? WL[n] : WR[n];
+        const double V = lt ? VL : VR, rho = lt ? rhoL : rhoR, k = lt ? kL : kR, Sk = lt ? SL : SR;
+        const double Sb = lt ? dmin(0.0, SL) : dmax(0.0, SR), p = W[IE];
+        const double dS = S - V, f = (Sk - V) * approx_rcp(Sk - S);
+        double AP = 0.0, BP = 0.0, rD = 0.0;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            AP = fma(W[IA + q], e.Ak[q], AP);
+            BP = fma(W[IA + q], e.Bk[q], BP);
+            rD = fma(W[q], e.Dk[q], rD);
+        }
+        const double E = fma(0.5 * rho, k, fma(AP, p, BP) + rD);
+        const double c = fma(Sb, f - 1.0, V);  // a transported component's flux is u c
+        const double m = rho * c, Sf = Sb * (f * dS);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            F[q] = W[q] * c;
+            F[IA + q] = W[IA + q] * c;
+        }
+#pragma unroll
+        for (int i = 0; i < D; ++i) F[IM + i] = W[IM + i] * m;
+#pragma unroll
+        for (int i = 0; i < D; ++i) F[IM + i] = (i == d) ? F[IM + i] + fma(Sf, rho, p) : F[IM + i];
+        F[IE] = fma(E, c, fma(Sf, fma(rho, S, p * approx_rcp(Sk - V)), p * V));
+        vel = c;
+    };
+    side(S >= 0.0, Fout, fnc[0]);
+    if (S == 0.0) {  // the mean of both sides
+        double F[N], v;
+        side(false, F, v);
+#pragma unroll
+        for (int i = 0; i < N; ++i) Fout[i] = 0.5 * (Fout[i] + F[i]);
+        fnc[0] = 0.5 * (fnc[0] + v);
+    }
+    cmax = dmax(cL + approx_sqrt(kL), cR + approx_sqrt(kR));
+}
+
+// Riemann flux of an N-phase face in the mixed form from FP32 face primitives; LIMIT: the consistent limiter
+// about the cell primitives cL, cR (component stride wstr) on either side first. NASG phases (whose covolume
+// is checked in every conversion) and the LLF / HLL solvers take the FP64 form's steps.
+template <class M, bool LIMIT, class PT, class Riemann>
+__device__ __forceinline__ void nphase_mixed_face(double* F, double* fnc, double& cm, const float* wL, const float* wR,
+                                                  const PT* cL, const PT* cR, int wstr, double dx, const Eos& e, int d,
+                                                  int id_k, bool hllc, Riemann general, unsigned int* err) {
+    bool nasg = false;
+#pragma unroll
+    for (int k = 0; k < M::NP; ++k) nasg |= (e.Ck[k] > 0.0);
+    if (hllc && !nasg) {
+        double WL[M::N], WR[M::N];
+        if constexpr (LIMIT) {
+            const double iden = 1.0 / (0.5 * dx);
+            nphase_limit_mixed<M>(WL, wL, cL, wstr, iden);
+            nphase_limit_mixed<M>(WR, wR, cR, wstr, -iden);
+        } else {
+#pragma unroll
+            for (int n = 0; n < M::N; ++n) {
+                WL[n] = wL[n];
+                WR[n] = wR[n];
+            }
+        }
+        nphase_hllc_mixed<M>(F, fnc, cm, WL, WR, e, d, id_k);
+        return;
+    }
+    double UL[M::N], UR[M::N], W[M::N];
+#pragma unroll
+    for (int n = 0; n < M::N; ++n) W[n] = wL[n];
+    M::prim2cons(UL, W, e, err);
+#pragma unroll
+    for (int n = 0; n < M::N; ++n) W[n] = wR[n];
+    M::prim2cons(UR, W, e, err);
+    if constexpr (LIMIT) {
+        M::consistent_limit(UL, cL, wstr, dx, 1, e, err);
+        M::consistent_limit(UR, cR, wstr, dx, -1, e, err);
+    }
+    general(UL, UR);
+}
 
 }  // namespace compas

@@ -2,23 +2,25 @@
 //
 // One CTA owns a tile of TX x TY x TZ cells. Per tile:
 //   1. the conserved state of the tile cells is read once and converted to primitives into shared
-//      memory (one Conservative2Primitive per cell instead of the reference's ~14 per face);
-//   2. per direction d: the 3-cell halo slabs on both sides of the tile in d are converted into a
-//      shared halo buffer; every face of the tile in d (T_d + 1 per line) is reconstructed (WENO5 in
-//      primitive variables on both sides, then Primitive2Conservative), solved by HLLC, and its flux
-//      and non-conservative face quantities are written to a shared face buffer; each cell then adds
-//      (F_hi - F_lo)/dx_d to its register accumulator, in the order x, y, z of the reference's
-//      divergence (include/Operators_FV/FVM_Divergence_D.H);
+//      memory (one Conservative2Primitive per cell instead of the reference's ~14 per face), with the
+//      3-cell halo slabs of all directions where they fit, else one direction's slabs at a time;
+//   2. per direction d, for all faces of the tile (T_d + 1 per line):
+//      a. reconstruction, one thread per line segment and component: the thread walks along the line and
+//         forms BOTH face values of each cell (WENO5; the two faces share the smoothness indicators and
+//         their ratios), written to a shared face buffer; WENO5B's bounded masses and volume fractions
+//         are formed together, one thread per cell;
+//      b. the Riemann flux, one thread per face, written over the face values it was formed from;
+//      c. each cell adds (F_hi - F_lo)/dx_d to its register accumulator, in the order x, y, z of the
+//         reference's divergence (include/Operators_FV/FVM_Divergence_D.H);
 //   3. the epilogue forms dUdt = -div F + NC terms, the RK3 stage combination and, for the
 //      six-equation model, the pressure relaxation, and writes the new state once.
 // Face fluxes never leave shared memory; the face wave speeds are max-reduced per CTA (warp
-// shuffles) into one atomic per CTA.
-//
-// The thread count NT is chosen so that the faces of one direction are an exact multiple of NT
-// (8^3 tile: 9*8*8 = 576 = 2 x 288 threads; 16^2 tile: 17*16 = 272 threads), which keeps every
-// face round full. Launch sites: source/Class_Compressible_PhaseField.cpp:3192-3250 (faces),
-// :3310-3386 (divergence and NC terms), :3937-4107 (stage combinations),
+// shuffles) into one atomic per CTA. Launch sites: source/Class_Compressible_PhaseField.cpp:3192-3250
+// (faces), :3310-3386 (divergence and NC terms), :3937-4107 (stage combinations),
 // source/Class_Compressible6Eq_PhaseField.cpp:437-474 (relaxation).
+//
+// The three-cell schemes and the THINC variant form their face states per face instead
+// (stage_tile_faces).
 #pragma once
 
 #include "physics.cuh"
@@ -71,6 +73,8 @@ struct StageArgs {
     int order;                 // tile traversal order (tile_coords): 0 x fastest, 1 bricks of tiles
     int tile_base;             // single-box kernels: first tile (order 0) and number of tiles of the launch
     int tile_count;            // (0: the whole box); a run of whole tile layers is a slab of the box
+    int map_ghosts;            // 0: ghost cells are read from Us; 1: a ghost cell is read as the valid cell its boundary
+    int lo_bc[3], hi_bc[3];    // condition maps it to (single-box domains), so Us needs no boundary fill
 };
 
 // Tile coordinates (in tiles) of the w-th CTA of a box of ntx x nty x ntz tiles. order 0: x fastest.
@@ -293,75 +297,307 @@ __device__ __forceinline__ void riemann(int id_riemann, double* Fout, double* fn
 
 namespace compas {
 
-// PF: the Phase-Field kernel, whose face buffer holds the model's NCPF non-conservative face terms.
-template <class M, int TX, int TY, int TZ, class PT = double, bool TMA = false, bool PF = false>
-struct TileShape {
-    static constexpr int D = M::D;
-    static constexpr int CELLS = TX * TY * TZ;
-    static constexpr int A0 = TY * TZ, A1 = TX * TZ, A2 = TX * TY;
-    static constexpr int AMAX = (D == 3) ? (A0 > A1 ? (A0 > A2 ? A0 : A2) : (A1 > A2 ? A1 : A2)) : (A0 > A1 ? A0 : A1);
-    // halo slab slot stride: padded by 8 cells in 3D so that the 4 slots a warp touches in one
-    // face round fall in different shared-memory banks
-    static constexpr int HS = (D == 3) ? AMAX + 8 : AMAX;
-    static constexpr int HALO = 6 * HS;
-    static constexpr int F0 = (TX + 1) * A0, F1 = (TY + 1) * A1, F2 = (TZ + 1) * A2;
-    static constexpr int FMAX = (D == 3) ? (F0 > F1 ? (F0 > F2 ? F0 : F2) : (F1 > F2 ? F1 : F2)) : (F0 > F1 ? F0 : F1);
-    static constexpr int NB = M::N + (PF ? M::NCPF : M::NC);
-    static constexpr size_t FB = sizeof(double) * (size_t)NB * FMAX;  // face buffer (FP64)
-    // Halo slab sets resident at once: D (every direction's slabs converted with the tile in step 1,
-    // one barrier per direction fewer) where the primitives and the face buffer fit two CTAs per SM
-    // (112 KB each), else 1 (the slabs of each direction converted before its faces, into one set).
-    static constexpr size_t kTwoCtaBytes = 112 * 1024;
-    static constexpr size_t pbytes(int nhs) { return sizeof(PT) * (size_t)M::N * (size_t)(CELLS + nhs * HALO); }
-    static constexpr int NHS = (!TMA && (pbytes(D) + 15) / 16 * 16 + FB <= kTwoCtaBytes) ? D : 1;
-    // primitives (type PT): component n of tile cell l at n * CSTR + l, of halo set h, slot s, slab
-    // cell t at n * CSTR + CELLS + h * HALO + s * HS + t (one component stride for tile and halo, so
-    // the stencil loads of a face differ only by compile-time offsets); then the face buffer
-    static constexpr int CSTR = CELLS + NHS * HALO;
-    static constexpr size_t PBYTES = pbytes(NHS);
-    static constexpr size_t FOFF = (PBYTES + 15) / 16 * 16;
-    static constexpr size_t FEND = FOFF + FB;
-    // TMA staging of one direction's two halo slabs (raw FP64 boxes of kTmaBoxX x 3 x T x N), placed
-    // at the next 128-byte boundary of the (runtime) shared-memory address, hence the 128-byte slack
-    static constexpr size_t SLAB = sizeof(double) * (size_t)kTmaBoxX * 3 * TX * M::N;
-    static constexpr size_t SMEM = TMA ? FEND + 128 + 2 * SLAB : FEND;
-};
-
 template <class M>
 __device__ __forceinline__ void load_cons(double* U, const double* base, const Grid& g, long long q) {
 #pragma unroll
     for (int n = 0; n < M::N; ++n) U[n] = base[n * g.S + q];
 }
 
-// SCHEME: 5 WENO5 on every primitive variable; 6 WENO5B (bounded masses and volume fractions,
-// plain WENO5 on the velocity and the pressure(s)); 2 GODUNOV / MUSCL in primitive variables, the
-// limiter a.muscl at run time.
-// MIX: false - plain FP64, the reference's arithmetic to the bit; true - mixed precision: the cell
-// primitives are recovered in FP64 (pressure from total energy) and kept in shared memory as FP32,
-// the reconstruction runs in FP32, the Riemann solver, divergence, stage accumulation and
-// relaxation in FP64.
-// VAR: kVarPlain - the hyperbolic right-hand side; kVarThinc - with THINC interface reconstruction
-// (FiniteVolume.THINC = 1); kVarPhaseField - the Phase-Field regularisation right-hand side (the
-// same face states, the regularisation flux of the face gradient a.gq instead of the Riemann flux;
-// FIVEEQS without non-conservative terms, SIXEQS with its phase-energy exchange).
-// The work of one CTA on tile `tile` of the box described by `a` (tiles numbered x fastest).
+// Source of coordinate x along d of a ghost cell (fill_cell's map: 0 periodic, 2 outflow, 3 / 4 mirrored with
+// the normal momentum odd, others mirrored with all momenta odd); odd collects the momenta to negate.
+__device__ __forceinline__ int ghost_source(int x, int n, int lo, int hi, int d, unsigned& odd) {
+    if (x >= 0 && x < n) return x;
+    const int code = (x < 0) ? lo : hi;
+    if (code == 0) return (x < 0) ? x + n : x - n;
+    if (code == 2) return (x < 0) ? 0 : n - 1;
+    odd ^= (code == 3 || code == 4) ? 1u << d : 7u;
+    return (x < 0) ? -1 - x : 2 * n - 1 - x;
+}
+
+// Conserved state of cell (i, j, k) of the stage's input; false outside the padded box. Interior cells take
+// no more than the range check; the ghost cells of a mapped input are those the boundary fill would write.
+template <class M>
+__device__ __forceinline__ bool load_state(double* U, const StageArgs& a, int i, int j, int k) {
+    const Grid& g = a.g;
+    unsigned odd = 0;
+    if (!((unsigned)i < (unsigned)g.n[0] && (unsigned)j < (unsigned)g.n[1] && (unsigned)k < (unsigned)g.n[2])) {
+        if (!g.padded(i, j, k)) return false;
+        if (a.map_ghosts) {
+            i = ghost_source(i, g.n[0], a.lo_bc[0], a.hi_bc[0], 0, odd);
+            j = ghost_source(j, g.n[1], a.lo_bc[1], a.hi_bc[1], 1, odd);
+            if (M::D == 3) k = ghost_source(k, g.n[2], a.lo_bc[2], a.hi_bc[2], 2, odd);
+        }
+    }
+    load_cons<M>(U, a.Us, g, g.at(i, j, k));
+    if (odd) {
+#pragma unroll
+        for (int c = 0; c < M::D; ++c)
+            if ((odd >> c) & 1u) U[M::IM + c] = -U[M::IM + c];
+    }
+    return true;
+}
+
+// Shared-memory layout of stage_tile_faces.
+template <class M, int TX, int TY, int TZ, class PT>
+struct TileShape {
+    static constexpr int D = M::D;
+    static constexpr int CELLS = TX * TY * TZ;
+    static constexpr int A0 = TY * TZ;  // lines of a direction (cubes and squares: the same for all)
+    // halo slab slot stride: padded by 8 cells in 3D so that the 4 slots a warp touches in one
+    // face round fall in different shared-memory banks
+    static constexpr int HS = (D == 3) ? A0 + 8 : A0;
+    static constexpr int HALO = 6 * HS;
+    static constexpr int FMAX = (TX + 1) * A0;
+    static constexpr int NB = M::N + M::NC;
+    static constexpr size_t FB = sizeof(double) * (size_t)NB * FMAX;  // face buffer (FP64)
+    // Halo slab sets resident at once: D (every direction's slabs converted with the tile in step 1,
+    // one barrier per direction fewer) where the primitives and the face buffer fit two CTAs per SM
+    // (112 KB each), else 1 (the slabs of each direction converted before its faces, into one set).
+    static constexpr size_t kTwoCtaBytes = 112 * 1024;
+    static constexpr size_t pbytes(int nhs) { return sizeof(PT) * (size_t)M::N * (size_t)(CELLS + nhs * HALO); }
+    static constexpr int NHS = ((pbytes(D) + 15) / 16 * 16 + FB <= kTwoCtaBytes) ? D : 1;
+    // primitives (type PT): component n of tile cell l at n * CSTR + l, of halo set h, slot s, slab
+    // cell t at n * CSTR + CELLS + h * HALO + s * HS + t (one component stride for tile and halo, so
+    // the stencil loads of a face differ only by compile-time offsets); then the face buffer
+    static constexpr int CSTR = CELLS + NHS * HALO;
+    static constexpr size_t FOFF = (pbytes(NHS) + 15) / 16 * 16;
+    static constexpr size_t SMEM = FOFF + FB;
+};
+
+// The new value of every cell of the tile from its divergence acc[r][.] (cell l = tid + r NT, x
+// fastest); prim(n, lx, ly, lz) is primitive n of a tile cell.
+template <class M, bool MIX, bool PFX, int TX, int TY, int TZ, int NT, int R, int NB, class P>
+__device__ __forceinline__ void stage_epilogue(const StageArgs& a, const double (&acc)[R][NB], int i0, int j0, int k0,
+                                               P prim) {
+    constexpr int N = M::N, D = M::D, CELLS = TX * TY * TZ;
+    constexpr bool NPH = (M::KIND == kModelFiveN);
+    constexpr bool SXN = (M::KIND == kModelSixN);
+    if (a.mode == kModeCmax) return;
+    const Grid& g = a.g;
+    unsigned int* err = a.err;
+    const int tid = threadIdx.x;
+    double dt = 0.0, ca = 1.0, cb = 0.0, cd = 1.0;
+    if (a.mode == kModeStage) {
+        dt = *a.dt;
+        if (a.stage == 1) { ca = 0.25; cb = 0.75; cd = 0.25; }
+        else if (a.stage == 2) { ca = 2.0 / 3.0; cb = 1.0 / 3.0; cd = 2.0 / 3.0; }
+    }
+    const double sdt = cd * dt;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int l = tid + r * NT;
+        if (l >= CELLS) continue;
+        const int lx = l % TX, ly = (l / TX) % TY, lz = l / (TX * TY);
+        const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
+        if (i >= g.n[0] || j >= g.n[1] || k >= g.n[2]) continue;
+        double W[N], L[N];
+        const long long q = g.at(i, j, k);
+        double Us[N];
+        load_cons<M>(Us, a.Us, g, q);
+        if constexpr (MIX) {
+            // masses and volume fraction exactly from the conserved state (FP64); the pressures
+            // of the non-conservative terms from the FP32 tile
+#pragma unroll
+            for (int n = 0; n < N; ++n) W[n] = prim(n, lx, ly, lz);
+            if constexpr (NPH || SXN) {
+#pragma unroll
+                for (int k = 0; k < M::NP; ++k) {
+                    W[M::IR + k] = Us[M::IR + k];
+                    W[M::IA + k] = Us[M::IA + k];
+                }
+            } else {
+                W[0] = Us[0];
+                W[1] = Us[1];
+                W[M::IA] = Us[M::IA];
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < N; ++n) W[n] = prim(n, lx, ly, lz);
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) L[n] = -acc[r][n];
+        if constexpr (PFX) {
+            if constexpr (M::KIND == kModelSix) {
+                // six-equation: the phase-energy exchange of the regularisation fluxes,
+                // u . (J_k rho_k . grad u) = div(J_k rho_k EK) - EK div(J_k rho_k)
+                // (include/Operators_Compressible6Eq_PhaseField/FVM_PhaseField_SurfaceIntegralNC_Compressible6Eq_PhaseField.H:15-85)
+                const double a1r1 = W[0], a2r2 = W[1];
+                const double rho = a1r1 + a2r2;
+                const double EK = 0.5 * ksum<D>(W + 2);
+                const double vg1 = acc[r][N + 2] - EK * acc[r][N];
+                const double vg2 = acc[r][N + 3] - EK * acc[r][N + 1];
+                const double x = (a1r1 / rho) * vg2 - (a2r2 / rho) * vg1;
+                L[M::IE1] = L[M::IE1] + x;
+                L[M::IE2] = L[M::IE2] + (-x);
+            }
+            // the five-equation model has no Phase-Field non-conservative terms
+            // (include/Operators_Compressible5Eq_PhaseField/FVM_PhaseField_SurfaceIntegralNC_Compressible5Eq_PhaseField.H)
+        } else if constexpr (M::KIND == kModelFive) {
+            // five-equation: alpha1 += phi1 (1 + K1) div u*
+            const double fac = M::kapila_factor(W, W, a.e, a.id_k, err);
+            L[M::IA] = L[M::IA] + fac * acc[r][N];
+        } else if constexpr (NPH) {
+            // N-phase five-equation: alpha_k += phi_k (1 + K_k) div u*
+            double fac[M::NP];
+            M::kapila_factors(fac, W, a.e, a.id_k, err);
+#pragma unroll
+            for (int k = 0; k < M::NP; ++k) L[M::IA + k] = L[M::IA + k] + fac[k] * acc[r][N];
+        } else if constexpr (SXN) {
+            // N-phase six-equation: alpha_k += alpha_k div u*, alpha_k rho_k e_k -= alpha_k p_k div u*
+            // (FVM_SurfaceIntegralNC_Compressible6Eq_IE_NPhase.H; acc holds +div u*, the reference
+            // subtracts alpha_k times its negative)
+            const double divv = acc[r][N];
+#pragma unroll
+            for (int k = 0; k < M::NP; ++k) {
+                L[M::IA + k] = L[M::IA + k] + W[M::IA + k] * divv;
+                L[M::IP + k] = L[M::IP + k] - W[M::IP + k] * divv;
+            }
+        } else {
+            // six-equation: phase energy exchange and alpha1 div u (FVM_SurfaceIntegralNC_Compressible6Eq.H)
+            const double divv = acc[r][N], dva1 = acc[r][N + 1], dva2 = acc[r][N + 2];
+            const double a1r1 = W[0], a2r2 = W[1];
+            const double rho = a1r1 + a2r2;
+            const double vg1 = dva1 - W[M::IE1] * divv;
+            const double vg2 = dva2 - W[M::IE2] * divv;
+            const double x = (a2r2 / rho) * vg1 - (a1r1 / rho) * vg2;
+            L[M::IE1] = L[M::IE1] + x;
+            L[M::IE2] = L[M::IE2] + (-x);
+            L[M::IA] = L[M::IA] + W[M::IA] * divv;
+        }
+        double out[N];
+        if (a.mode == kModeDudt) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) out[n] = L[n];
+        } else {
+            if (a.stage == 0) {
+#pragma unroll
+                for (int n = 0; n < N; ++n) out[n] = 1.0 * Us[n] + sdt * L[n];
+            } else {
+                double U0[N];
+                load_cons<M>(U0, a.U0, g, q);
+#pragma unroll
+                for (int n = 0; n < N; ++n) {
+                    double v = ca * Us[n] + cb * U0[n];
+                    out[n] = v + sdt * L[n];
+                }
+            }
+            if constexpr (M::KIND == kModelSix) {
+                if (a.relax) relax_pressure<D, MIX>(out, a.e, a.trace, err);
+            } else if constexpr (SXN) {
+                if (a.relax) M::relax(out, a.e, a.trace, err);
+            }
+            bool bad = false;
+#pragma unroll
+            for (int n = 0; n < N; ++n) bad |= isnan(out[n]);
+            if (bad) flag_error(err, COMPAS_B200_ERR_NAN);
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) a.Uout[n * g.S + q] = out[n];
+    }
+}
+
+// CTA max of the face wave speeds -> one atomic.
+template <int NT>
+__device__ __forceinline__ void cta_cmax(unsigned long long* cmax, double v) {
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __shared__ double wmax[32];
+    const int w = tid >> 5, lane = tid & 31;
+    if (lane == 0) wmax[w] = v;
+    __syncthreads();
+    if (tid == 0) {
+        double m = 0.0;
+        for (int q = 0; q < (NT + 31) / 32; ++q) m = dmax(m, wmax[q]);
+        // non-negative doubles order like their bit patterns; a NaN speed propagates as the max
+        atomicMax(cmax, (unsigned long long)__double_as_longlong(m));
+    }
+}
+
+// Conserved upwind state of a mixed Riemann solver from the FP32 face primitives.
+template <class M>
+struct MixedState {
+    const float* wL;
+    const float* wR;
+    const Eos& e;
+    __device__ __forceinline__ void operator()(bool left, double* U) const {
+        float w[M::N];
+#pragma unroll
+        for (int n = 0; n < M::N; ++n) w[n] = left ? wL[n] : wR[n];
+        M::prim2cons_f32(U, w, e);
+    }
+};
+
+// Riemann flux of the two-phase models in the mixed form from FP32 face primitives; state(left, U) gives
+// the conserved face states.
+template <class M, class State>
+__device__ __forceinline__ void mixed_riemann(int id_riemann, double* F, double* fnc, float& cm, const float* wL,
+                                              const float* wR, const Eos& e, int d, int id_k, State state) {
+    if (id_riemann != 2) {
+        double UL[M::N], UR[M::N];
+        state(true, UL);
+        state(false, UR);
+        llf_hll_mixed<M>(id_riemann, F, fnc, cm, UL, UR, wL, wR, e, d, id_k);
+    } else if constexpr (M::KIND == kModelFive) {
+        fiveeq_hllc_mixed<M::D>(F, fnc, cm, wL, wR, e, d, id_k, state);
+    } else {
+        sixeq_hllc_mixed<M::D>(F, fnc, cm, wL, wR, e, d, state);
+    }
+}
+
+// The face wave speed alone (the t = 0 pass): the operations the Riemann solvers form it with, FP64 form.
+template <class M>
+__device__ __forceinline__ double face_speed(const double* UL, const double* UR, const Eos& e, int id_k, unsigned int* err) {
+    double q[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        double W[M::N], c;
+        M::cons2prim(W, s ? UR : UL, e, err);
+        if constexpr (M::KIND == kModelSix) c = M::sound_speed(W, e, err);
+        else c = M::sound_speed(W, e, id_k, err);
+        q[s] = c + sqrt(ksum<M::D>(W + M::IM));
+    }
+    return dmax(q[0], q[1]);
+}
+
+// The same of a two-phase model in the mixed form.
+template <class M>
+__device__ __forceinline__ float face_speed_mixed(const float* wL, const float* wR, const Eos& e, int id_k) {
+    float q[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const float* w = s ? wR : wL;
+        float c, k = __fmaf_rn(w[2], w[2], w[3] * w[3]);
+        if (M::D == 3) k = __fmaf_rn(w[4], w[4], k);
+        if constexpr (M::KIND == kModelSix) c = sixeq_c_f32<M::D>(w, e);
+        else c = fiveeq_c_f32<M::D>(w, e, id_k);
+        q[s] = c + sqrt_ftz(k);
+    }
+    return fmaxf(q[0], q[1]);
+}
+
+// The covolume status of a face state (two-phase models): the check of the FP64 conversions.
+template <class M>
+__device__ __forceinline__ void covolume_check(const float* w, const Eos& e, unsigned int* err) {
+    nasg_xi(w[M::IA], w[0], e.C1, err);
+    nasg_xi(1.0 - (double)w[M::IA], w[1], e.C2, err);
+}
+
+// The work of one CTA on tile `tile` for the schemes whose face states are formed per face: the
+// three-cell schemes (SCHEME 2: GODUNOV / MUSCL / WENO3 in primitive variables, the limiter a.muscl at
+// run time) and THINC (VAR kVarThinc: the faces at an interface, the others WENO5 / WENO5B). One thread
+// per face reconstructs both states and solves; the rest as stage_tile.
 template <class M, int SCHEME, bool MIX, int VAR, int TX, int TY, int TZ, int NT>
-__device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double* smem_d, const TmaMaps* tm = nullptr) {
+__device__ __forceinline__ void stage_tile_faces(const StageArgs& a, int tile, double* smem_d) {
     static_assert(TX == TY && (M::D == 2 ? TZ == 1 : TZ == TX), "tiles are cubes (squares in 2D)");
     constexpr bool TH = (VAR == kVarThinc);
-    constexpr bool PFX = (VAR == kVarPhaseField);
-    constexpr bool TMA = (VAR == kVarTma);
-    static_assert(!TMA || (M::D == 3 && MIX), "TMA halo staging: the 3D mixed form");
-    static_assert(!PFX || M::KIND != kModelFiveN, "the Phase-Field kernel is the two-phase models'");
-    static_assert(M::KIND != kModelFiveN || !TH, "FIVEEQS_NPHASE runs without THINC");
-    static_assert(M::KIND != kModelSixN || VAR == kVarPlain,
-                  "SIXEQS_IE_NPHASE: the plain hyperbolic right-hand side");
-    static_assert(SCHEME != 2 || (VAR == kVarPlain && !TH), "GODUNOV / MUSCL: the plain right-hand side");
+    static_assert((SCHEME == 2) != TH, "the three-cell schemes, or THINC");
+    static_assert(!TH || M::KIND == kModelFive || M::KIND == kModelSix, "THINC: the two-phase models");
     constexpr bool NPH = (M::KIND == kModelFiveN);
     constexpr bool SXN = (M::KIND == kModelSixN);
     using PT = typename std::conditional<MIX, float, double>::type;
-    using T = TileShape<M, TX, TY, TZ, PT, TMA, PFX>;
-    constexpr int N = M::N, NC = PFX ? M::NCPF : M::NC, D = M::D, NB = T::NB;
+    using T = TileShape<M, TX, TY, TZ, PT>;
+    constexpr int N = M::N, NC = M::NC, D = M::D, NB = T::NB;
     constexpr int CELLS = T::CELLS, HALO = T::HALO, FMAX = T::FMAX;
     constexpr int R = (CELLS + NT - 1) / NT;
 
@@ -382,13 +618,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
     const int k0 = tiz * TZ;
     const int tid = threadIdx.x;
     unsigned int* err = a.err;
-    __shared__ uint64_t tma_bar;
-    double* stg = nullptr;  // TMA staging: low slab, then high slab
-    if constexpr (TMA) {
-        stg = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_d) + T::FEND + 127) & ~uintptr_t(127));
-        if (tid == 0) mbar_init(&tma_bar, 1);  // visible to all after the barrier that ends step 1
-    }
-
     // 1. tile cells and the x-direction halo slabs -> primitives, read as whole rows of TX + 6 cells
     // (coalesced), the tile cells into Pint and the halo cells into the x slabs of halo set 0; with
     // NHS = D also the y (and z) halo slabs, into halo sets 1 (and 2), in the same loop
@@ -422,8 +651,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
         const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
         double U[N];
         PT W[N];
-        if (g.padded(i, j, k)) {
-            load_cons<M>(U, a.Us, g, g.at(i, j, k));
+        if (load_state<M>(U, a, i, j, k)) {
             if constexpr (MIX) M::cons2prim_f32(W, U, a.e);
             else M::cons2prim(W, U, a.e, nullptr);
         } else {
@@ -444,48 +672,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
         constexpr int Ad = T::A0;
         constexpr int Ta = TX;
         // 2a. halo slabs of direction d -> primitives (the x slabs came with the rows of step 1)
-        if constexpr (TMA) {
-            if (d > 0) {
-                // the slabs were staged by TMA during the previous direction's faces (phase d - 1).
-                // A wait that runs out sets the status bit and waits once more (bounded) for the copy
-                // in flight; if that runs out too, the whole CTA leaves the tile without reading the
-                // staging buffer or writing any output (a timed-out tile leaves its cells unwritten)
-                bool lost = false;
-                if (!mbar_wait_bounded(&tma_bar, (unsigned)(d - 1), 1 << 20)) {
-                    flag_error(err, COMPAS_B200_ERR_TIMEOUT);
-                    lost = !mbar_wait_bounded(&tma_bar, (unsigned)(d - 1), 1 << 20);
-                }
-                if (__syncthreads_or(lost)) return;
-                const int offx = (i0 + g.ng) - ((i0 + g.ng - 1) & ~1);
-                for (int h = tid; h < 6 * Ad; h += NT) {
-                    const int slot = h / Ad, t = h % Ad;
-                    const int pos = (slot < 3) ? slot - 3 : Td + slot - 3;
-                    const int ta = t % Ta, tb = t / Ta;
-                    const int b = (slot < 3) ? slot : slot - 3;
-                    const double* sl = stg + ((slot < 3) ? 0 : T::SLAB / sizeof(double));
-                    // box element (x, y, z) of component n: n*(10*3*8) + z*(10*Y) + y*10 + x
-                    const int e0 = (d == 1) ? (ta + offx) + kTmaBoxX * b + kTmaBoxX * 3 * tb
-                                            : (ta + offx) + kTmaBoxX * tb + kTmaBoxX * Ta * b;
-                    int lx, ly, lz;
-                    if (d == 1) { lx = ta; ly = pos; lz = tb; }
-                    else { lx = ta; ly = tb; lz = pos; }
-                    double U[N];
-                    PT W[N];
-                    if (g.padded(i0 + lx, j0 + ly, k0 + lz)) {
-#pragma unroll
-                        for (int n = 0; n < N; ++n) U[n] = sl[n * (kTmaBoxX * 3 * Ta) + e0];
-                        M::cons2prim_f32(W, U, a.e);
-                    } else {
-#pragma unroll
-                        for (int n = 0; n < N; ++n) W[n] = 0;
-                    }
-#pragma unroll
-                    for (int n = 0; n < N; ++n) Phal[n * CSTR + slot * T::HS + t] = W[n];
-                }
-            }
-        }
         // with one halo set, the slabs of d > 0 are converted here (d = 0 came with the rows of step 1)
-        for (int h = (d == 0 || TMA || NHS == D) ? 6 * Ad : tid; h < 6 * Ad; h += NT) {
+        for (int h = (d == 0 || NHS == D) ? 6 * Ad : tid; h < 6 * Ad; h += NT) {
             const int slot = h / Ad, t = h % Ad;
             const int pos = (slot < 3) ? slot - 3 : Td + slot - 3;
             const int ta = t % Ta, tb = t / Ta;
@@ -496,8 +684,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
             const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
             double U[N];
             PT W[N];
-            if (g.padded(i, j, k)) {
-                load_cons<M>(U, a.Us, g, g.at(i, j, k));
+            if (load_state<M>(U, a, i, j, k)) {
                 if constexpr (MIX) M::cons2prim_f32(W, U, a.e);
                 else M::cons2prim(W, U, a.e, nullptr);
             } else {
@@ -519,23 +706,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
         constexpr int EF = TS + 1;
         const int NF = EF * T::A0;
         const double dxd = (d == 0) ? g.dx[0] : (d == 1 ? g.dx[1] : g.dx[2]);
-        if constexpr (TMA) {
-            // stage the next direction's two halo slabs while this direction's faces are computed;
-            // the staging was last read before the barrier above
-            if (tid == 0 && d + 1 < D) {
-                fence_proxy_async_smem();
-                mbar_arrive_expect_tx(&tma_bar, (unsigned)(2 * T::SLAB));
-                const int xs = (i0 + g.ng - 1) & ~1;  // even: an 8-byte element start on a 16-byte boundary
-                double* hi = stg + T::SLAB / sizeof(double);
-                if (d == 0) {
-                    tma_load_4d(stg, &tm->y, &tma_bar, xs, j0 + g.ng - 3, k0 + g.gz, 0);
-                    tma_load_4d(hi, &tm->y, &tma_bar, xs, j0 + g.ng + TY, k0 + g.gz, 0);
-                } else {
-                    tma_load_4d(stg, &tm->z, &tma_bar, xs, j0 + g.ng, k0 + g.gz - 3, 0);
-                    tma_load_4d(hi, &tm->z, &tma_bar, xs, j0 + g.ng, k0 + g.gz + TZ, 0);
-                }
-            }
-        }
         for (int f = tid; f < NF; f += NT) {
             int fd, ta, tb;
             if (d == 0) {
@@ -591,19 +761,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                                                       UR, err);
             if constexpr (!MIX) {
                 if (!thinc_face) {
-                    if constexpr (SCHEME == 6 && (NPH || SXN)) {
-                        double rf[M::NP], af[M::NP];
-                        auto rl = [&](int k, int s) { return (double)smem[off[s] + (M::IR + k) * str[s]]; };
-                        auto al_ = [&](int k, int s) { return (double)smem[off[s] + (M::IA + k) * str[s]]; };
-                        bounded_phases<M::NP, 5, double>(rl, al_, 1, rf, af);
-#pragma unroll
-                        for (int k = 0; k < M::NP; ++k) { WfL[M::IR + k] = rf[k]; WfL[M::IA + k] = af[k]; }
-                        auto rr = [&](int k, int s) { return (double)smem[off[s + 1] + (M::IR + k) * str[s + 1]]; };
-                        auto ar_ = [&](int k, int s) { return (double)smem[off[s + 1] + (M::IA + k) * str[s + 1]]; };
-                        bounded_phases<M::NP, 5, double>(rr, ar_, -1, rf, af);
-#pragma unroll
-                        for (int k = 0; k < M::NP; ++k) { WfR[M::IR + k] = rf[k]; WfR[M::IA + k] = af[k]; }
-                    } else if constexpr (SCHEME == 6) {
+                    if constexpr (SCHEME == 6) {
                         double r1[6], r2[6], al[6];
 #pragma unroll
                         for (int s = 0; s < 6; ++s) {
@@ -641,39 +799,26 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                     }
                     M::prim2cons(UL, WfL, a.e, err);
                     M::prim2cons(UR, WfR, a.e, err);
-                    if constexpr (NPH && SCHEME != 6) if (SCHEME != 2 || a.muscl != 11) {
-                        // N-phase WENO5 / three-cell schemes: the consistent limiter about the stencil
-                        // centres f-1 and f (WENO5B bounds its face values instead)
+                    if constexpr (NPH) if (a.muscl != 11) {
+                        // N-phase: the consistent limiter about the stencil centres f-1 and f (WENO3B bounds
+                        // its face values instead)
                         M::consistent_limit(UL, smem + off[2], str[2], dxd, 1, a.e, err);
                         M::consistent_limit(UR, smem + off[3], str[3], dxd, -1, a.e, err);
                     }
-                    if constexpr (SXN && SCHEME == 2) if (a.muscl >= 1 && a.muscl < 10) {
+                    if constexpr (SXN) if (a.muscl >= 1 && a.muscl < 10) {
                         // N-phase six-equation: the consistent limiter after MUSCL only
                         M::consistent_limit(UL, smem + off[2], str[2], dxd, 1, a.e, err);
                         M::consistent_limit(UR, smem + off[3], str[3], dxd, -1, a.e, err);
                     }
                 }
-                if constexpr (PFX) {
-                    pf_face_fluxes<M, MIX>(F, fnc, UL, UR, pf_face_gq(a, d, gi, gj, gk), a.e, a.pf_phasic, a.pf_hll,
-                                           err);
-                    cm = 0.0;
-                } else {
-                    riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
-                }
+                riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
             } else {
                 float wL[N], wR[N];
                 if (thinc_face) {
                     M::cons2prim_f32(wL, UL, a.e);
                     M::cons2prim_f32(wR, UR, a.e);
                 } else {
-                    if constexpr (SCHEME == 6 && (NPH || SXN)) {
-                        auto rl = [&](int k, int s) { return (float)smem[off[s] + (M::IR + k) * str[s]]; };
-                        auto al_ = [&](int k, int s) { return (float)smem[off[s] + (M::IA + k) * str[s]]; };
-                        bounded_phases<M::NP, 5, float>(rl, al_, 1, wL + M::IR, wL + M::IA);
-                        auto rr = [&](int k, int s) { return (float)smem[off[s + 1] + (M::IR + k) * str[s + 1]]; };
-                        auto ar_ = [&](int k, int s) { return (float)smem[off[s + 1] + (M::IA + k) * str[s + 1]]; };
-                        bounded_phases<M::NP, 5, float>(rr, ar_, -1, wR + M::IR, wR + M::IA);
-                    } else if constexpr (SCHEME == 6) {
+                    if constexpr (SCHEME == 6) {
                         float r1[6], r2[6], al[6];
 #pragma unroll
                         for (int s = 0; s < 6; ++s) {
@@ -716,11 +861,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                     }
                     M::prim2cons(UL, WfL, a.e, err);
                     M::prim2cons(UR, WfR, a.e, err);
-                    if constexpr (NPH && SCHEME != 6) if (SCHEME != 2 || a.muscl != 11) {
+                    if constexpr (NPH) if (a.muscl != 11) {
                         M::consistent_limit(UL, smem + off[2], str[2], dxd, 1, a.e, err);
                         M::consistent_limit(UR, smem + off[3], str[3], dxd, -1, a.e, err);
                     }
-                    if constexpr (SXN && SCHEME == 2) if (a.muscl >= 1 && a.muscl < 10) {
+                    if constexpr (SXN) if (a.muscl >= 1 && a.muscl < 10) {
                         M::consistent_limit(UL, smem + off[2], str[2], dxd, 1, a.e, err);
                         M::consistent_limit(UR, smem + off[3], str[3], dxd, -1, a.e, err);
                     }
@@ -730,17 +875,10 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                     riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
                 } else {
                     float cmf;
-                    if constexpr (PFX) {
-                        pf_face_fluxes<M, MIX>(F, fnc, UL, UR, pf_face_gq(a, d, gi, gj, gk), a.e, a.pf_phasic,
-                                               a.pf_hll, err);
-                        cmf = 0.0f;
-                    } else if (a.riemann != 2) {
-                        llf_hll_mixed<M>(a.riemann, F, fnc, cmf, UL, UR, wL, wR, a.e, d, a.id_k);
-                    } else if constexpr (M::KIND == kModelFive) {
-                        fiveeq_hllc_mixed<D>(F, fnc, cmf, UL, UR, wL, wR, a.e, d, a.id_k);
-                    } else {
-                        sixeq_hllc_mixed<D>(F, fnc, cmf, UL, UR, wL, wR, a.e, d);
-                    }
+                    mixed_riemann<M>(a.riemann, F, fnc, cmf, wL, wR, a.e, d, a.id_k, [&](bool left, double* U) {
+#pragma unroll
+                        for (int n = 0; n < N; ++n) U[n] = left ? UL[n] : UR[n];
+                    });
                     cm = cmf;
                 }
             }
@@ -781,143 +919,533 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
     }
 
     // 3. epilogue
-    if (a.mode != kModeCmax) {
-        double dt = 0.0, ca = 1.0, cb = 0.0, cd = 1.0;
-        if (a.mode == kModeStage) {
-            dt = *a.dt;
-            if (a.stage == 1) { ca = 0.25; cb = 0.75; cd = 0.25; }
-            else if (a.stage == 2) { ca = 2.0 / 3.0; cb = 1.0 / 3.0; cd = 2.0 / 3.0; }
+    stage_epilogue<M, MIX, false, TX, TY, TZ, NT, R, NB>(a, acc, i0, j0, k0, [&](int n, int lx, int ly, int lz) {
+        return (double)Pint[n * CSTR + lx + TX * (ly + TY * lz)];
+    });
+
+    // CTA max of the face wave speeds -> one atomic
+    if (a.cmax) cta_cmax<NT>(a.cmax, cmax_local);
+}
+
+// Shared-memory layout of stage_tile and its work split. In 2D the primitives are one array of the tile
+// with its x and y halos (rows of TS + 6, pitch 23); in 3D the tile cells (row pitch 9, plane pitch 72)
+// and, beside them, NHS sets of six halo planes. The pitches put the 32 lines a warp walks along x or y in
+// different banks. Component n of every cell is CSTR further.
+//
+// Face buffer: [slot of the face][lines], component stride FSTR, one 8-byte entry per component: the two
+// FP32 face values and then, in place, the FP64 flux (mixed form); or the FP64 left values, the right values N
+// components further, and then the flux over the left ones. Where that buffer of 2N doubles a face leaves no
+// room for CTAS CTAs per SM, the lines of a direction are taken in two halves (NCH = 2).
+template <class M, int TS, class PT, bool TMA, bool PF, int CTAS>
+struct ReconShape {
+    static constexpr int D = M::D, N = M::N;
+    static constexpr bool MIX = std::is_same<PT, float>::value;
+    static constexpr int LINES = (D == 3) ? TS * TS : TS;
+    static constexpr int CELLS = LINES * TS;
+    static constexpr int NB = N + (PF ? M::NCPF : M::NC);
+    static constexpr size_t kBudget = 224 * 1024 / CTAS;  // shared memory of one CTA
+    static constexpr int FCOMP = MIX ? NB : (2 * N > NB ? 2 * N : NB);
+    static constexpr int pitch(int lc) { return (D == 3) ? lc + 2 : lc + 1; }
+    static constexpr size_t fbytes(int lc) { return sizeof(double) * (size_t)FCOMP * (TS + 1) * pitch(lc); }
+    static constexpr int PX = (D == 3) ? TS + 1 : TS + 7;
+    static constexpr int PZ = PX * TS;                    // 3D plane pitch
+    static constexpr int TCELLS = (D == 3) ? PZ * TS : PX * (TS + 6);
+    static constexpr int HALO = 6 * LINES;                // a set of halo planes (3D)
+    static constexpr int cstr(int nhs) { return (D == 3) ? TCELLS + nhs * HALO : (TCELLS + 31) / 32 * 32 + 16; }
+    static constexpr size_t pbytes(int nhs) { return (sizeof(PT) * (size_t)N * cstr(nhs) + 15) / 16 * 16; }
+    // the lines of a direction in one pass where the face buffer fits, else in two halves
+    static constexpr int NCH = (D == 3 && pbytes(1) + fbytes(LINES) > kBudget) ? 2 : 1;
+    static constexpr int LC = LINES / NCH;      // lines of a pass
+    static constexpr int LS = pitch(LC);        // pitch of a face slot
+    static constexpr int FSTR = (TS + 1) * LS;  // component stride of the face buffer
+    static constexpr size_t FB = fbytes(LC);
+    // every direction's halo planes converted with the tile where they fit, else one direction's at a time
+    static constexpr int NHS = (D == 2 || (!TMA && pbytes(D) + FB <= kBudget)) ? D : 1;
+    static constexpr int CSTR = cstr(NHS);
+    static constexpr size_t FOFF = pbytes(NHS);
+    static constexpr size_t FEND = FOFF + FB;
+    // TMA staging of one direction's two halo slabs (raw FP64 boxes of kTmaBoxX x 3 x T x N), placed
+    // at the next 128-byte boundary of the (runtime) shared-memory address, hence the 128-byte slack
+    static constexpr size_t SLAB = sizeof(double) * (size_t)kTmaBoxX * 3 * TS * N;
+    static constexpr size_t SMEM = TMA ? FEND + 128 + 2 * SLAB : FEND;
+
+    // offset of cell `pos` of line t along d (pos -3 .. TS + 2)
+    __device__ static __forceinline__ int base(int d, int t) {
+        if constexpr (D == 2) return (d == 0) ? 3 + PX * (t + 3) : (t + 3) + PX * 3;
+        else return (d == 0) ? PX * (t % TS) + PZ * (t / TS) : (d == 1) ? t % TS + PZ * (t / TS) : t % TS + PX * (t / TS);
+    }
+    __device__ static __forceinline__ int stride(int d) {
+        if constexpr (D == 2) return (d == 0) ? 1 : PX;
+        else return (d == 0) ? 1 : (d == 1) ? PX : PZ;
+    }
+    __device__ static __forceinline__ int halo(int d, int t) { return TCELLS + ((NHS == 1) ? 0 : d) * HALO + t; }
+    __device__ static __forceinline__ int cell(int base, int stride, int halo, int pos) {
+        if constexpr (D == 2) return base + pos * stride;
+        else return (pos < 0) ? halo + (pos + 3) * LINES : (pos < TS) ? base + pos * stride : halo + (pos - TS + 3) * LINES;
+    }
+};
+
+// Cells of a line segment that one thread walks, so that the items of a pass fill the CTA's threads evenly:
+// the smallest rounds x (cells + start), `start` standing for the beginning of a segment in tenths of a cell.
+__host__ __device__ constexpr int segment_cells(int items_per_seg, int cells, int nt, int start) {
+    int best = cells, cost = 1 << 30;
+    for (int sc = 2; sc <= cells; ++sc) {
+        const int segs = (cells + sc - 1) / sc;
+        const int rounds = (items_per_seg * segs + nt - 1) / nt;
+        if (rounds * (10 * sc + start) < cost) {
+            cost = rounds * (10 * sc + start);
+            best = sc;
         }
-        const double sdt = cd * dt;
+    }
+    return best;
+}
+
+__device__ __forceinline__ void weno5_cell(float f0, float f1, float f2, float f3, float f4, float& vp, float& vm) {
+    weno5_both_f32(f0, f1, f2, f3, f4, vp, vm);
+}
+__device__ __forceinline__ void weno5_cell(double f0, double f1, double f2, double f3, double f4, double& vp, double& vm) {
+    weno5_both(f0, f1, f2, f3, f4, vp, vm);
+}
+
+// Step 2a: the face values of the lines [line0, line0 + LC) along d into the face buffer Fb.
+template <class M, int SCHEME, class T, class PT, int TS, int NT>
+__device__ __forceinline__ void reconstruct_lines(const PT* prim, double* Fb, int d, int line0, int nl_a, int nl_b) {
+    constexpr int N = M::N, LC = T::LC, LS = T::LS, FSTR = T::FSTR, CSTR = T::CSTR, NCELL = TS + 2;
+    constexpr bool F32 = std::is_same<PT, float>::value;
+    constexpr bool NPH = (M::KIND == kModelFiveN || M::KIND == kModelSixN);
+    constexpr int NB0 = (SCHEME == 6) ? weno5b_plain_lo<M>() : 0;
+    constexpr int NB1 = (SCHEME == 6) ? weno5b_plain_hi<M>() : N;
+    const int tid = threadIdx.x;
+    const int sd = T::stride(d);
+    // value v of component n at face slot f of line tl, side 0 left, 1 right
+    auto put = [&](int n, int f, int tl, int side, PT v) {
+        if constexpr (F32) reinterpret_cast<float*>(Fb)[2 * (n * FSTR + f * LS + tl) + side] = v;
+        else Fb[(n + side * N) * FSTR + f * LS + tl] = v;
+    };
+    // lines outside the box (ragged tiles) are skipped: their transverse coordinates are (a, b)
+    auto line_valid = [&](int t) { return t % TS < nl_a && (T::D == 2 || t / TS < nl_b); };
+
+    int first = 0;
+    if constexpr (SCHEME == 6) {
+        // bounded masses and volume fractions: one thread per cell -1 .. TS
+        constexpr int ITEMS = LC * NCELL;
+        for (int it = tid; it < ITEMS; it += NT) {
+            const int tl = it % LC, t = line0 + tl, i = it / LC - 1;
+            if (!line_valid(t)) continue;
+            const int b = T::base(d, t), h = T::halo(d, t);
+            const PT* p[5];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int l = tid + r * NT;
-            if (l >= CELLS) continue;
-            const int lx = l % TX, ly = (l / TX) % TY, lz = l / (TX * TY);
-            const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
-            if (i >= g.n[0] || j >= g.n[1] || k >= g.n[2]) continue;
-            double W[N], L[N];
-            const long long q = g.at(i, j, k);
-            double Us[N];
-            load_cons<M>(Us, a.Us, g, q);
-            if constexpr (MIX) {
-                // masses and volume fraction exactly from the conserved state (FP64); the pressures
-                // of the non-conservative terms from the FP32 tile
-#pragma unroll
-                for (int n = 0; n < N; ++n) W[n] = Pint[n * CSTR + l];
-                if constexpr (NPH || SXN) {
-#pragma unroll
-                    for (int k = 0; k < M::NP; ++k) {
-                        W[M::IR + k] = Us[M::IR + k];
-                        W[M::IA + k] = Us[M::IA + k];
-                    }
-                } else {
-                    W[0] = Us[0];
-                    W[1] = Us[1];
-                    W[M::IA] = Us[M::IA];
-                }
-            } else {
-#pragma unroll
-                for (int n = 0; n < N; ++n) W[n] = Pint[n * CSTR + l];
-            }
-#pragma unroll
-            for (int n = 0; n < N; ++n) L[n] = -acc[r][n];
-            if constexpr (PFX) {
-                if constexpr (M::KIND == kModelSix) {
-                    // six-equation: the phase-energy exchange of the regularisation fluxes,
-                    // u . (J_k rho_k . grad u) = div(J_k rho_k EK) - EK div(J_k rho_k)
-                    // (include/Operators_Compressible6Eq_PhaseField/FVM_PhaseField_SurfaceIntegralNC_Compressible6Eq_PhaseField.H:15-85)
-                    const double a1r1 = W[0], a2r2 = W[1];
-                    const double rho = a1r1 + a2r2;
-                    const double EK = 0.5 * ksum<D>(W + 2);
-                    const double vg1 = acc[r][N + 2] - EK * acc[r][N];
-                    const double vg2 = acc[r][N + 3] - EK * acc[r][N + 1];
-                    const double x = (a1r1 / rho) * vg2 - (a2r2 / rho) * vg1;
-                    L[M::IE1] = L[M::IE1] + x;
-                    L[M::IE2] = L[M::IE2] + (-x);
-                }
-                // the five-equation model has no Phase-Field non-conservative terms
-                // (include/Operators_Compressible5Eq_PhaseField/FVM_PhaseField_SurfaceIntegralNC_Compressible5Eq_PhaseField.H)
-            } else if constexpr (M::KIND == kModelFive) {
-                // five-equation: alpha1 += phi1 (1 + K1) div u*
-                const double fac = M::kapila_factor(W, W, a.e, a.id_k, err);
-                L[M::IA] = L[M::IA] + fac * acc[r][N];
-            } else if constexpr (NPH) {
-                // N-phase five-equation: alpha_k += phi_k (1 + K_k) div u*
-                double fac[M::NP];
-                M::kapila_factors(fac, W, a.e, a.id_k, err);
-#pragma unroll
-                for (int k = 0; k < M::NP; ++k) L[M::IA + k] = L[M::IA + k] + fac[k] * acc[r][N];
-            } else if constexpr (SXN) {
-                // N-phase six-equation: alpha_k += alpha_k div u*, alpha_k rho_k e_k -= alpha_k p_k div u*
-                // (FVM_SurfaceIntegralNC_Compressible6Eq_IE_NPhase.H; acc holds +div u*, the reference
-                // subtracts alpha_k times its negative)
-                const double divv = acc[r][N];
+            for (int s = 0; s < 5; ++s) p[s] = prim + T::cell(b, sd, h, i - 2 + s);
+            if constexpr (NPH) {
+                PT rp[M::NP], ap[M::NP], rm[M::NP], am[M::NP];
+                bounded_phases_both<M::NP, 5, PT>([&](int k, int s) { return p[s][(M::IR + k) * CSTR]; },
+                                                  [&](int k, int s) { return p[s][(M::IA + k) * CSTR]; }, rp, ap, rm, am);
 #pragma unroll
                 for (int k = 0; k < M::NP; ++k) {
-                    L[M::IA + k] = L[M::IA + k] + W[M::IA + k] * divv;
-                    L[M::IP + k] = L[M::IP + k] - W[M::IP + k] * divv;
-                }
-            } else {
-                // six-equation: phase energy exchange and alpha1 div u (FVM_SurfaceIntegralNC_Compressible6Eq.H)
-                const double divv = acc[r][N], dva1 = acc[r][N + 1], dva2 = acc[r][N + 2];
-                const double a1r1 = W[0], a2r2 = W[1];
-                const double rho = a1r1 + a2r2;
-                const double vg1 = dva1 - W[M::IE1] * divv;
-                const double vg2 = dva2 - W[M::IE2] * divv;
-                const double x = (a2r2 / rho) * vg1 - (a1r1 / rho) * vg2;
-                L[M::IE1] = L[M::IE1] + x;
-                L[M::IE2] = L[M::IE2] + (-x);
-                L[M::IA] = L[M::IA] + W[M::IA] * divv;
-            }
-            double out[N];
-            if (a.mode == kModeDudt) {
-#pragma unroll
-                for (int n = 0; n < N; ++n) out[n] = L[n];
-            } else {
-                if (a.stage == 0) {
-#pragma unroll
-                    for (int n = 0; n < N; ++n) out[n] = 1.0 * Us[n] + sdt * L[n];
-                } else {
-                    double U0[N];
-                    load_cons<M>(U0, a.U0, g, q);
-#pragma unroll
-                    for (int n = 0; n < N; ++n) {
-                        double v = ca * Us[n] + cb * U0[n];
-                        out[n] = v + sdt * L[n];
+                    if (i < TS) {
+                        put(M::IR + k, i + 1, tl, 0, rp[k]);
+                        put(M::IA + k, i + 1, tl, 0, ap[k]);
+                    }
+                    if (i >= 0) {
+                        put(M::IR + k, i, tl, 1, rm[k]);
+                        put(M::IA + k, i, tl, 1, am[k]);
                     }
                 }
-                if constexpr (M::KIND == kModelSix) {
-                    if (a.relax) relax_pressure<D, MIX>(out, a.e, a.trace, err);
-                } else if constexpr (SXN) {
-                    if (a.relax) M::relax(out, a.e, a.trace, err);
+            } else {
+                PT r1[5], r2[5], al[5], Wp[3], Wm[3];
+#pragma unroll
+                for (int s = 0; s < 5; ++s) {
+                    r1[s] = p[s][0];
+                    r2[s] = p[s][CSTR];
+                    al[s] = p[s][M::IA * CSTR];
                 }
-                bool bad = false;
-#pragma unroll
-                for (int n = 0; n < N; ++n) bad |= isnan(out[n]);
-                if (bad) flag_error(err, COMPAS_B200_ERR_NAN);
+                if constexpr (F32) weno5b_masses_both_f32(r1, r2, al, Wp, Wm);
+                else weno5b_masses_both(r1, r2, al, 1.0 / 12.0, Wp, Wm, 2);
+                if (i < TS) {
+                    put(0, i + 1, tl, 0, Wp[0]);
+                    put(1, i + 1, tl, 0, Wp[1]);
+                    put(M::IA, i + 1, tl, 0, Wp[2]);
+                }
+                if (i >= 0) {
+                    put(0, i, tl, 1, Wm[0]);
+                    put(1, i, tl, 1, Wm[1]);
+                    put(M::IA, i, tl, 1, Wm[2]);
+                }
             }
+        }
+        first = ITEMS % NT;  // the threads that had no item in the last round start the next loop
+    }
+    // plain WENO5: one thread per (component, segment, line)
+    constexpr int NPL = NB1 - NB0;
+    // (FP32 in 3D walks whole lines: unrolled, every offset is then known at compile time)
+    constexpr int SEG = (T::D == 3 && F32) ? NCELL : segment_cells(LC * NPL, NCELL, NT, F32 ? 20 : 3);
+    constexpr int NSEG = (NCELL + SEG - 1) / SEG;
+    constexpr int ITEMS = LC * NPL * NSEG;
+    for (int it = (tid >= first) ? tid - first : tid + NT - first; it < ITEMS; it += NT) {
+        const int tl = it % LC, t = line0 + tl, q = it / LC;
+        const int n = NB0 + q % NPL;
+        const int i0 = (NSEG == 1) ? -1 : (q / NPL) * SEG - 1;  // first cell of the segment
+        if (!line_valid(t)) continue;
+        const int b = T::base(d, t), h = T::halo(d, t);
+        const PT* p = prim + n * CSTR;
+        auto ld = [&](int pos) { return p[T::cell(b, sd, h, pos)]; };
+        PT f0 = ld(i0 - 2), f1 = ld(i0 - 1), f2 = ld(i0), f3 = ld(i0 + 1);
+        PT vl = 0;  // left value of the current cell's low face, from the cell before
+        // FP32: unrolled, so that squares and products of differences carry over from cell to cell. FP64: a
+        // cell is some 400 instructions (12 divisions); rolled, the loop stays in the instruction cache.
+        constexpr int UNROLL = F32 ? SEG : 1;
+#pragma unroll UNROLL
+        for (int j = 0; j < SEG; ++j) {
+            const int i = i0 + j;
+            if (NSEG * SEG > NCELL && i > TS) break;  // the last segment may be shorter
+            const PT f4 = ld(i + 2);
+            PT vp, vm;
+            weno5_cell(f0, f1, f2, f3, f4, vp, vm);
+            if constexpr (F32) {
+                if (i >= 0) {
+                    if (j > 0) reinterpret_cast<float2*>(Fb)[n * FSTR + i * LS + tl] = make_float2(vl, vm);
+                    else put(n, i, tl, 1, vm);
+                }
+                if (j == SEG - 1 && i < TS) put(n, i + 1, tl, 0, vp);
+                vl = vp;
+            } else {
+                if (i >= 0) put(n, i, tl, 1, vm);
+                if (i < TS) put(n, i + 1, tl, 0, vp);
+            }
+            f0 = f1;
+            f1 = f2;
+            f2 = f3;
+            f3 = f4;
+        }
+    }
+}
+
+// SCHEME: 5 WENO5 on every primitive variable; 6 WENO5B (bounded masses and volume fractions,
+// plain WENO5 on the velocity and the pressure(s)).
+// MIX: false - plain FP64, the reference's arithmetic to the bit; true - mixed precision: the cell
+// primitives are recovered in FP64 (pressure from total energy) and kept in shared memory as FP32,
+// the reconstruction runs in FP32, the Riemann solver, divergence, stage accumulation and
+// relaxation in FP64.
+// VAR: kVarPlain - the hyperbolic right-hand side; kVarTma - the same with the halo slabs staged by TMA;
+// kVarPhaseField - the Phase-Field regularisation right-hand side (the
+// same face states, the regularisation flux of the face gradient a.gq instead of the Riemann flux;
+// FIVEEQS without non-conservative terms, SIXEQS with its phase-energy exchange).
+// The work of one CTA on tile `tile` of the box described by `a` (tiles numbered x fastest).
+//
+// What bounds it: instruction issue, not memory (DRAM traffic is the algorithmic bytes). Forming both face
+// values of a cell at once halves the smoothness indicators and, in FP64, takes 12 divisions instead of 18.
+template <class M, int SCHEME, bool MIX, int VAR, int TX, int TY, int TZ, int NT, int CTAS>
+__device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double* smem_d, const TmaMaps* tm = nullptr) {
+    static_assert(TX == TY && (M::D == 2 ? TZ == 1 : TZ == TX), "tiles are cubes (squares in 2D)");
+    static_assert(SCHEME == 5 || SCHEME == 6, "the fifth-order schemes");
+    constexpr bool PFX = (VAR == kVarPhaseField);
+    constexpr bool TMA = (VAR == kVarTma);
+    static_assert(!TMA || (M::D == 3 && MIX), "TMA halo staging: the 3D mixed form");
+    static_assert(!PFX || M::KIND == kModelFive || M::KIND == kModelSix, "the Phase-Field kernel is the two-phase models'");
+    constexpr bool NPH = (M::KIND == kModelFiveN);
+    constexpr bool SXN = (M::KIND == kModelSixN);
+    using PT = typename std::conditional<MIX, float, double>::type;
+    constexpr int TS = TX;
+    using T = ReconShape<M, TS, PT, TMA, PFX, CTAS>;
+    constexpr int N = M::N, NC = PFX ? M::NCPF : M::NC, D = M::D, NB = T::NB;
+    constexpr int CELLS = T::CELLS, LINES = T::LINES, LC = T::LC, LS = T::LS, FSTR = T::FSTR;
+    constexpr int CSTR = T::CSTR, NHS = T::NHS, EF = TS + 1;
+    constexpr int R = (CELLS + NT - 1) / NT;
+
+    PT* prim = reinterpret_cast<PT*>(smem_d);
+    double* Fb = reinterpret_cast<double*>(reinterpret_cast<char*>(smem_d) + T::FOFF);
+
+    const Grid& g = a.g;
+    const int ntx = (g.n[0] + TX - 1) / TX;
+    const int nty = (g.n[1] + TY - 1) / TY;
+    const int ntz = (g.n[2] + TZ - 1) / TZ;
+    int tix, tiy, tiz;
+    tile_coords(tile, ntx, nty, ntz, a.order, D, tix, tiy, tiz);
+    const int i0 = tix * TX;
+    const int j0 = tiy * TY;
+    const int k0 = tiz * TZ;
+    const int tid = threadIdx.x;
+    unsigned int* err = a.err;
+    __shared__ uint64_t tma_bar;
+    double* stg = nullptr;  // TMA staging: low slab, then high slab
+    if constexpr (TMA) {
+        stg = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_d) + T::FEND + 127) & ~uintptr_t(127));
+        if (tid == 0) mbar_init(&tma_bar, 1);  // visible to all after the barrier that ends step 1
+    }
+
+    // conserved state of cell (lx, ly, lz) of the tile's frame -> primitives at offset dst
+    auto convert = [&](int lx, int ly, int lz, int dst) {
+        const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
+        double U[N];
+        PT W[N];
+        if (load_state<M>(U, a, i, j, k)) {
+            if constexpr (MIX) M::cons2prim_f32(W, U, a.e);
+            else M::cons2prim(W, U, a.e, nullptr);
+        } else {
 #pragma unroll
-            for (int n = 0; n < N; ++n) a.Uout[n * g.S + q] = out[n];
+            for (int n = 0; n < N; ++n) W[n] = 0;
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) prim[n * CSTR + dst] = W[n];
+    };
+
+    // 1. tile cells and the x halo, read as whole rows of TX + 6 cells (coalesced), and with NHS = D the y
+    // (and z) halo slabs in the same loop
+    constexpr int RX = TX + 6;
+    constexpr int ROWS = RX * TY * TZ;
+    constexpr int ITEMS = ROWS + ((NHS == D) ? (D - 1) * 6 * LINES : 0);
+    for (int l = tid; l < ITEMS; l += NT) {
+        int lx, ly, lz, dst;
+        if (l < ROWS) {
+            lx = l % RX - 3;
+            ly = (l / RX) % TY;
+            lz = l / (RX * TY);
+            if constexpr (D == 2) dst = lx + 3 + T::PX * (ly + 3);
+            else dst = T::cell(T::base(0, ly + TS * lz), 1, T::halo(0, ly + TS * lz), lx);
+        } else {
+            const int h = l - ROWS;
+            const int dd = 1 + h / (6 * LINES);
+            const int hh = h - (dd - 1) * 6 * LINES;
+            const int slot = hh / LINES, t = hh % LINES;
+            const int pos = (slot < 3) ? slot - 3 : TX + slot - 3;
+            lx = t % TX;
+            if (dd == 1) { ly = pos; lz = t / TX; }
+            else { ly = t / TX; lz = pos; }
+            if constexpr (D == 2) dst = lx + 3 + T::PX * (ly + 3);
+            else dst = T::halo(dd, t) + slot * LINES;
+        }
+        convert(lx, ly, lz, dst);
+    }
+
+    double acc[R][NB];
+    double cmax_local = 0.0;
+
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) {
+        // with one halo set, the slabs of d > 0 (the x slabs came with the rows of step 1)
+        if constexpr (TMA) {
+            if (d > 0) {
+                // the slabs were staged by TMA during the previous direction's faces (phase d - 1).
+                // A wait that runs out sets the status bit and waits once more (bounded) for the copy
+                // in flight; if that runs out too, the whole CTA leaves the tile without reading the
+                // staging buffer or writing any output (a timed-out tile leaves its cells unwritten)
+                bool lost = false;
+                if (!mbar_wait_bounded(&tma_bar, (unsigned)(d - 1), 1 << 20)) {
+                    flag_error(err, COMPAS_B200_ERR_TIMEOUT);
+                    lost = !mbar_wait_bounded(&tma_bar, (unsigned)(d - 1), 1 << 20);
+                }
+                if (__syncthreads_or(lost)) return;
+                const int offx = (i0 + g.ng) - ((i0 + g.ng - 1) & ~1);
+                for (int h = tid; h < 6 * LINES; h += NT) {
+                    const int slot = h / LINES, t = h % LINES;
+                    const int pos = (slot < 3) ? slot - 3 : TS + slot - 3;
+                    const int ta = t % TS, tb = t / TS;
+                    const int b = (slot < 3) ? slot : slot - 3;
+                    const double* sl = stg + ((slot < 3) ? 0 : T::SLAB / sizeof(double));
+                    // box element (x, y, z) of component n: n*(10*3*8) + z*(10*Y) + y*10 + x
+                    const int e0 = (d == 1) ? (ta + offx) + kTmaBoxX * b + kTmaBoxX * 3 * tb
+                                            : (ta + offx) + kTmaBoxX * tb + kTmaBoxX * TS * b;
+                    const int ly = (d == 1) ? pos : tb, lz = (d == 1) ? tb : pos;
+                    double U[N];
+                    PT W[N];
+                    if (g.padded(i0 + ta, j0 + ly, k0 + lz)) {
+#pragma unroll
+                        for (int n = 0; n < N; ++n) U[n] = sl[n * (kTmaBoxX * 3 * TS) + e0];
+                        M::cons2prim_f32(W, U, a.e);
+                    } else {
+#pragma unroll
+                        for (int n = 0; n < N; ++n) W[n] = 0;
+                    }
+#pragma unroll
+                    for (int n = 0; n < N; ++n) prim[n * CSTR + T::halo(d, t) + slot * LINES] = W[n];
+                }
+            }
+        } else if constexpr (NHS != D) {
+            for (int h = (d == 0) ? 6 * LINES : tid; h < 6 * LINES; h += NT) {
+                const int slot = h / LINES, t = h % LINES;
+                const int pos = (slot < 3) ? slot - 3 : TS + slot - 3;
+                convert(t % TS, (d == 1) ? pos : t / TS, (d == 1) ? t / TS : pos, T::halo(d, t) + slot * LINES);
+            }
+        }
+        const double dxd = (d == 0) ? g.dx[0] : (d == 1 ? g.dx[1] : g.dx[2]);
+        const double idxd = 1.0 / dxd;
+        // lines of the tile inside the box, per transverse direction
+        const int nl_a = (d == 0) ? g.n[1] - j0 : g.n[0] - i0;
+        const int nl_b = (d == 2) ? g.n[1] - j0 : g.n[2] - k0;
+
+#pragma unroll 1
+        for (int ch = 0; ch < T::NCH; ++ch) {
+            const int line0 = ch * LC;
+            // the primitives are written, and the previous pass has read its fluxes
+            __syncthreads();
+            if constexpr (TMA) {
+                // stage the next direction's two halo slabs while this direction's faces are computed;
+                // the staging was last read before the barrier above
+                if (tid == 0 && d + 1 < D) {
+                    fence_proxy_async_smem();
+                    mbar_arrive_expect_tx(&tma_bar, (unsigned)(2 * T::SLAB));
+                    const int xs = (i0 + g.ng - 1) & ~1;  // even: an 8-byte element start on a 16-byte boundary
+                    double* hi = stg + T::SLAB / sizeof(double);
+                    if (d == 0) {
+                        tma_load_4d(stg, &tm->y, &tma_bar, xs, j0 + g.ng - 3, k0 + g.gz, 0);
+                        tma_load_4d(hi, &tm->y, &tma_bar, xs, j0 + g.ng + TY, k0 + g.gz, 0);
+                    } else {
+                        tma_load_4d(stg, &tm->z, &tma_bar, xs, j0 + g.ng, k0 + g.gz - 3, 0);
+                        tma_load_4d(hi, &tm->z, &tma_bar, xs, j0 + g.ng, k0 + g.gz + TZ, 0);
+                    }
+                }
+            }
+            // 2a. face values
+            reconstruct_lines<M, SCHEME, T, PT, TS, NT>(prim, Fb, d, line0, nl_a, nl_b);
+            __syncthreads();
+
+            // 2b. fluxes, one thread per face, in place over the face values
+            for (int f = tid; f < EF * LC; f += NT) {
+                const int fd = f / LC, tl = f % LC, t = line0 + tl;
+                const int ta = t % TS, tb = t / TS;
+                int gi = i0, gj = j0, gk = k0;
+                if (d == 0) { gi += fd; gj += ta; gk += tb; }
+                else if (d == 1) { gi += ta; gj += fd; gk += tb; }
+                else { gi += ta; gj += tb; gk += fd; }
+                const int gd = (d == 0) ? gi : (d == 1 ? gj : gk);
+                const int nd = (d == 0) ? g.n[0] : (d == 1 ? g.n[1] : g.n[2]);
+                if (gd > nd || ta >= nl_a || (D == 3 && tb >= nl_b)) continue;
+                double* fb = Fb + fd * LS + tl;
+                double F[N], fnc[NC], cm;
+                if constexpr (!MIX) {
+                    double UL[N], UR[N];
+                    {
+                        double W[N];
+#pragma unroll
+                        for (int n = 0; n < N; ++n) W[n] = fb[n * FSTR];
+                        M::prim2cons(UL, W, a.e, err);
+#pragma unroll
+                        for (int n = 0; n < N; ++n) W[n] = fb[(N + n) * FSTR];
+                        M::prim2cons(UR, W, a.e, err);
+                    }
+                    if constexpr (NPH && SCHEME == 5) {
+                        // N-phase WENO5: the consistent limiter about the stencil centres f-1 and f (WENO5B
+                        // bounds its face values instead)
+                        const int b = T::base(d, t), h = T::halo(d, t), sd = T::stride(d);
+                        M::consistent_limit(UL, prim + T::cell(b, sd, h, fd - 1), CSTR, dxd, 1, a.e, err);
+                        M::consistent_limit(UR, prim + T::cell(b, sd, h, fd), CSTR, dxd, -1, a.e, err);
+                    }
+                    if constexpr (PFX) {
+                        pf_face_fluxes<M, MIX>(F, fnc, UL, UR, pf_face_gq(a, d, gi, gj, gk), a.e, a.pf_phasic, a.pf_hll,
+                                               err);
+                        cm = 0.0;
+                    } else {
+                        if constexpr (!SXN) if (a.mode == kModeCmax) {
+                            cm = face_speed<M>(UL, UR, a.e, a.id_k, err);
+                            if (fd < TS && gd < nd) cmax_local = dmax(cm, cmax_local);
+                            continue;
+                        }
+                        riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
+                    }
+                } else {
+                    float wL[N], wR[N];
+#pragma unroll
+                    for (int n = 0; n < N; ++n) {
+                        const float2 w = reinterpret_cast<const float2*>(fb)[n * FSTR];
+                        wL[n] = w.x;
+                        wR[n] = w.y;
+                    }
+                    if constexpr (NPH) {
+                        // FP32 reconstruction, FP64 limiter (WENO5; WENO5B bounds its face values instead) and
+                        // Riemann solver
+                        const int b = T::base(d, t), h = T::halo(d, t), sd = T::stride(d);
+                        nphase_mixed_face<M, SCHEME == 5>(
+                            F, fnc, cm, wL, wR, prim + T::cell(b, sd, h, fd - 1), prim + T::cell(b, sd, h, fd), CSTR, dxd,
+                            a.e, d, a.id_k, a.riemann == 2, [&](const double* UL, const double* UR) {
+                                riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
+                            }, err);
+                    } else if constexpr (SXN || PFX) {
+                        double UL[N], UR[N];
+                        {
+                            double W[N];
+#pragma unroll
+                            for (int n = 0; n < N; ++n) W[n] = wL[n];
+                            M::prim2cons(UL, W, a.e, err);
+#pragma unroll
+                            for (int n = 0; n < N; ++n) W[n] = wR[n];
+                            M::prim2cons(UR, W, a.e, err);
+                        }
+                        if constexpr (PFX) {
+                            pf_face_fluxes<M, MIX>(F, fnc, UL, UR, pf_face_gq(a, d, gi, gj, gk), a.e, a.pf_phasic,
+                                                   a.pf_hll, err);
+                            cm = 0.0;
+                        } else {
+                            riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
+                        }
+                    } else {
+                        if (a.e.C1 > 0.0 || a.e.C2 > 0.0) {
+                            covolume_check<M>(wL, a.e, err);
+                            covolume_check<M>(wR, a.e, err);
+                        }
+                        float cmf;
+                        if (a.mode == kModeCmax) {
+                            cm = face_speed_mixed<M>(wL, wR, a.e, a.id_k);
+                            if (fd < TS && gd < nd) cmax_local = dmax(cm, cmax_local);
+                            continue;
+                        }
+                        mixed_riemann<M>(a.riemann, F, fnc, cmf, wL, wR, a.e, d, a.id_k, MixedState<M>{wL, wR, a.e});
+                        cm = cmf;
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < N; ++n) fb[n * FSTR] = F[n];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) fb[(N + c) * FSTR] = fnc[c];
+                if (fd < TS && gd < nd) cmax_local = dmax(cm, cmax_local);
+            }
+            if (a.mode == kModeCmax) continue;  // wave speeds only
+            __syncthreads();
+
+            // 2c. divergence contribution of direction d: (F+ - F-)/dx as the reference divides (FP64 form);
+            // times the reciprocal of dx in the mixed form (an FP64 division per term dominates otherwise)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int l = tid + r * NT;
+                if (l >= CELLS) continue;
+                const int lx = l % TX, ly = (l / TX) % TY, lz = l / (TX * TY);
+                const int t = (d == 0) ? ly + TS * lz : lx + TS * ((d == 1) ? lz : ly);
+                const int pos = (d == 0) ? lx : (d == 1) ? ly : lz;
+                if (T::NCH > 1 && t / LC != ch) continue;
+                const double* fb = Fb + pos * LS + (t - line0);
+#pragma unroll
+                for (int c = 0; c < NB; ++c) {
+                    const double df = fb[c * FSTR + LS] - fb[c * FSTR];
+                    if constexpr (MIX) {
+                        acc[r][c] = (d == 0) ? df * idxd : fma(df, idxd, acc[r][c]);
+                    } else {
+                        const double tt = df / dxd;
+                        acc[r][c] = (d == 0) ? tt : acc[r][c] + tt;
+                    }
+                }
+            }
         }
     }
 
-    // CTA max of the face wave speeds -> one atomic
-    if (a.cmax) {
-        double v = cmax_local;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-        __shared__ double wmax[32];
-        const int w = tid >> 5, lane = tid & 31;
-        if (lane == 0) wmax[w] = v;
-        __syncthreads();
-        if (tid == 0) {
-            double m = 0.0;
-            for (int q = 0; q < (NT + 31) / 32; ++q) m = dmax(m, wmax[q]);
-            // non-negative doubles order like their bit patterns; a NaN speed propagates as the max
-            atomicMax(a.cmax, (unsigned long long)__double_as_longlong(m));
-        }
-    }
+    // 3. epilogue
+    stage_epilogue<M, MIX, PFX, TX, TY, TZ, NT, R, NB>(a, acc, i0, j0, k0, [&](int n, int lx, int ly, int lz) {
+        return (double)prim[n * CSTR + ((D == 2) ? lx + 3 + T::PX * (ly + 3) : lx + T::PX * ly + T::PZ * lz)];
+    });
+    if (a.cmax) cta_cmax<NT>(a.cmax, cmax_local);
+}
+
+// The tile routine of a scheme and variant.
+template <class M, int SCHEME, bool MIX, int VAR, int TX, int TY, int TZ, int NT, int CTAS>
+__device__ __forceinline__ void run_tile(const StageArgs& a, int tile, double* smem_d, const TmaMaps* tm = nullptr) {
+    if constexpr (SCHEME == 2 || VAR == kVarThinc) stage_tile_faces<M, SCHEME, MIX, VAR, TX, TY, TZ, NT>(a, tile, smem_d);
+    else stage_tile<M, SCHEME, MIX, VAR, TX, TY, TZ, NT, CTAS>(a, tile, smem_d, tm);
+}
+
+// Dynamic shared memory of run_tile.
+template <class M, int SCHEME, bool MIX, int VAR, int TS, int TZ, int CTAS>
+constexpr size_t tile_smem() {
+    using PT = typename std::conditional<MIX, float, double>::type;
+    if constexpr (SCHEME == 2 || VAR == kVarThinc) return TileShape<M, TS, TS, TZ, PT>::SMEM;
+    else return ReconShape<M, TS, PT, VAR == kVarTma, VAR == kVarPhaseField, CTAS>::SMEM;
 }
 
 // One box: one CTA per tile.
@@ -925,7 +1453,7 @@ template <class M, int SCHEME, bool MIX, int VAR, int TX, int TY, int TZ, int NT
 __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
     if (a.done && *a.done) return;
     extern __shared__ double smem_d[];
-    stage_tile<M, SCHEME, MIX, VAR, TX, TY, TZ, NT>(a, a.tile_base + blockIdx.x, smem_d);
+    run_tile<M, SCHEME, MIX, VAR, TX, TY, TZ, NT, MINB>(a, a.tile_base + blockIdx.x, smem_d);
 }
 
 // One box with the halo slabs staged by TMA (the tensor maps of a.Us are kernel parameters).
@@ -933,7 +1461,7 @@ template <class M, int SCHEME, bool MIX, int TX, int TY, int TZ, int NT, int MIN
 __global__ void __launch_bounds__(NT, MINB) stage_kernel_tma(StageArgs a, const __grid_constant__ TmaMaps tm) {
     if (a.done && *a.done) return;
     extern __shared__ __align__(128) double smem_d[];
-    stage_tile<M, SCHEME, MIX, kVarTma, TX, TY, TZ, NT>(a, a.tile_base + blockIdx.x, smem_d, &tm);
+    stage_tile<M, SCHEME, MIX, kVarTma, TX, TY, TZ, NT, MINB>(a, a.tile_base + blockIdx.x, smem_d, &tm);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -967,7 +1495,8 @@ struct ListArgs {
     int mode;
     int stage;
     int order;                    // tile traversal order inside each box (tile_coords)
-};
+    int map_ghosts;               // the boxes are single-box domains whose ghost cells are read through their boundary
+};                                // conditions (StageArgs::map_ghosts)
 
 __device__ __forceinline__ int find_box(const int* off, int nb, int w) {
     int lo = 0, hi = nb - 1;
@@ -1022,10 +1551,15 @@ __global__ void __launch_bounds__(NT, MINB) stage_list_kernel(ListArgs L) {
             sa.pf_hll = 0;
             sa.muscl = B.muscl;
             sa.riemann = B.riemann;
-            for (int d = 0; d < 3; ++d) sa.gq[d] = nullptr;
+            sa.map_ghosts = L.map_ghosts;
+            for (int d = 0; d < 3; ++d) {
+                sa.gq[d] = nullptr;
+                sa.lo_bc[d] = B.lo_bc[d];
+                sa.hi_bc[d] = B.hi_bc[d];
+            }
         }
         __syncthreads();
-        stage_tile<M, SCHEME, MIX, kVarPlain, TX, TY, TZ, NT>(sa, w - L.tile_off[b], smem_d);
+        run_tile<M, SCHEME, MIX, kVarPlain, TX, TY, TZ, NT, MINB>(sa, w - L.tile_off[b], smem_d);
     }
 }
 
