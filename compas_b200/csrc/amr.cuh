@@ -22,10 +22,12 @@
 
 namespace compas {
 
-// ghost cell copied from a valid cell of a box of the same level (periodic images included)
+// ghost cell copied from a valid cell of a box of the same level (periodic images, and the mirror or
+// outflow image of a cell outside the domain, included), with the components whose sign the boundary flips
 struct AmrSame {
     int db, sb;
     long long dq, sq;
+    unsigned odd;
 };
 // ghost cell interpolated from the coarse level: stencil cells C, C-e0, C+e0, C-e1, C+e1 (, C-e2, C+e2)
 // with, per stencil cell, the coarse box, the padded index and the components whose value changes
@@ -36,13 +38,8 @@ struct AmrInterp {
     int cb[7];
     long long cq[7];
     unsigned odd[7];
-    int par;  // bit d set: the fine cell is the upper child along d (offset +1/4)
-};
-// ghost cell outside the domain along one direction: mirror / extrapolation within the same box
-struct AmrBc {
-    int b;
-    long long dq, sq;
-    unsigned odd;
+    int par;       // bit d set: the fine cell is the upper child along d (offset +1/4)
+    unsigned flip; // a cell outside the domain: the components its image within the domain has with the other sign
 };
 // coarse-fine face between an uncovered coarse cell and the fine region
 struct AmrCf {
@@ -89,8 +86,6 @@ struct AmrLevelH {
     long long n_same = 0;
     AmrInterp* d_interp = nullptr;
     long long n_interp = 0;
-    AmrBc* d_bc[3] = {nullptr, nullptr, nullptr};
-    long long n_bc[3] = {0, 0, 0};
     // as the fine level of the pair (l-1, l): coarse-fine faces, registers, reflux groups
     AmrCf* d_cf = nullptr;
     int n_cf = 0;
@@ -108,69 +103,107 @@ struct AmrBufs {
     const long long* S;        // component stride of each box
 };
 
-__global__ void amr_same_kernel(const AmrSame* t, long long n, AmrBufs B, int dk, int sk, int N) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const AmrSame e = t[q];
-        double* dst = B.p[e.db * 4 + dk];
-        const double* src = B.p[e.sb * 4 + sk];
-        const long long Sd = B.S[e.db], Ss = B.S[e.sb];
-        for (int c = 0; c < N; ++c) dst[c * Sd + e.dq] = src[c * Ss + e.sq];
-    }
+// Most components of a model (the N-phase six-equation model with three phases in 3D has 13).
+constexpr int kAmrMaxComp = 16;
+
+__device__ __forceinline__ void amr_copy_cell(const AmrSame& e, const AmrBufs& B, int k, int N) {
+    double* dst = B.p[e.db * 4 + k] + e.dq;
+    const double* src = B.p[e.sb * 4 + k] + e.sq;
+    const long long Sd = B.S[e.db], Ss = B.S[e.sb];
+    double v[kAmrMaxComp];
+#pragma unroll
+    for (int c = 0; c < kAmrMaxComp; ++c)
+        if (c < N) v[c] = src[c * Ss];
+#pragma unroll
+    for (int c = 0; c < kAmrMaxComp; ++c)
+        if (c < N) dst[c * Sd] = ((e.odd >> c) & 1u) ? -1.0 * v[c] : v[c];
 }
 
-// mode 0: coarse new data, 1: coarse old data, 2: alpha old + beta new
-__device__ __forceinline__ double amr_coarse(const AmrBufs& B, int cb, long long cq, int c, int knew, int kold, int mode,
-                                             double alpha, double beta) {
-    const long long S = B.S[cb];
-    if (mode == 0) return B.p[cb * 4 + knew][c * S + cq];
-    if (mode == 1) return B.p[cb * 4 + kold][c * S + cq];
-    return alpha * B.p[cb * 4 + kold][c * S + cq] + beta * B.p[cb * 4 + knew][c * S + cq];
-}
-
+// mode 0: coarse new data, 1: coarse old data, 2: alpha old + beta new.
 // pc: amr.Interpolater = pc_interp (the parent's value, AMReX PCInterp); else lincc_interp as restated in the
 // file header: per direction the central slopes of all components, one monotonized-central factor shared
-// by the components, u_f = u_c + sum_d +-1/4 slope_d
-__global__ void amr_interp_kernel(const AmrInterp* t, long long n, AmrBufs B, int dk, int knew, int kold, int mode,
-                                  double alpha, double beta, int N, int D, int pc) {
-    constexpr int NMAX = 2 * COMPAS_B200_MAX_PHASES + 4;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const AmrInterp& e = t[q];
-        double* dst = B.p[e.db * 4 + dk];
-        const long long Sd = B.S[e.db];
-        auto val = [&](int s, int c) {
-            const double v = amr_coarse(B, e.cb[s], e.cq[s], c, knew, kold, mode, alpha, beta);
-            return ((e.odd[s] >> c) & 1u) ? -1.0 * v : 1.0 * v;
-        };
-        double u[NMAX];
-        for (int c = 0; c < N; ++c) u[c] = val(0, c);
-        for (int d = 0; d < (pc ? 0 : D); ++d) {
-            double dcs[NMAX];
-            double sf = 1.0;
-            for (int c = 0; c < N; ++c) {
-                const double uc = val(0, c);
-                const double um = val(1 + 2 * d, c), up = val(2 + 2 * d, c);
-                const double dc = 0.5 * (up - um), df = 2.0 * (up - uc), db = 2.0 * (uc - um);
+// by the components, u_f = u_c + sum_d +-1/4 slope_d. The components are loaded together (N predicated loads in
+// flight), not one after the other.
+__device__ __forceinline__ void amr_interp_cell(const AmrInterp& e, const AmrBufs& B, int dk, int knew, int kold, int mode,
+                                                double alpha, double beta, int N, int D, int pc) {
+    auto load = [&](int s, double* v) {
+        const int b = e.cb[s];
+        const long long S = B.S[b], q = e.cq[s];
+        const unsigned odd = e.odd[s];
+        const double* pn = B.p[b * 4 + knew] + q;
+        const double* po = B.p[b * 4 + kold] + q;
+#pragma unroll
+        for (int c = 0; c < kAmrMaxComp; ++c)
+            if (c < N) {
+                double x = (mode == 0) ? pn[c * S] : po[c * S];
+                if (mode == 2) x = alpha * x + beta * pn[c * S];
+                v[c] = ((odd >> c) & 1u) ? -1.0 * x : x;
+            }
+    };
+    double uc[kAmrMaxComp], u[kAmrMaxComp];
+    load(0, uc);
+#pragma unroll
+    for (int c = 0; c < kAmrMaxComp; ++c) u[c] = uc[c];
+    for (int d = 0; d < (pc ? 0 : D); ++d) {
+        double um[kAmrMaxComp], up[kAmrMaxComp];
+        load(1 + 2 * d, um);
+        load(2 + 2 * d, up);
+        double sf = 1.0;
+#pragma unroll
+        for (int c = 0; c < kAmrMaxComp; ++c)
+            if (c < N) {
+                const double dc = 0.5 * (up[c] - um[c]), df = 2.0 * (up[c] - uc[c]), db = 2.0 * (uc[c] - um[c]);
                 double sx = (df * db >= 0.0) ? dmin(fabs(df), fabs(db)) : 0.0;
                 sx = copysign(1.0, dc) * dmin(sx, fabs(dc));
                 if (dc != 0.0) sf = dmin(sf, sx / dc);
-                dcs[c] = dc;
+                um[c] = dc;
             }
-            const double off = ((e.par >> d) & 1) ? 0.25 : -0.25;
-            for (int c = 0; c < N; ++c) u[c] = u[c] + off * (dcs[c] * sf);
-        }
-        for (int c = 0; c < N; ++c) dst[c * Sd + e.dq] = u[c];
+        const double off = ((e.par >> d) & 1) ? 0.25 : -0.25;
+#pragma unroll
+        for (int c = 0; c < kAmrMaxComp; ++c)
+            if (c < N) u[c] = u[c] + off * (um[c] * sf);
     }
+    double* dst = B.p[e.db * 4 + dk] + e.dq;
+    const long long Sd = B.S[e.db];
+#pragma unroll
+    for (int c = 0; c < kAmrMaxComp; ++c)
+        if (c < N) dst[c * Sd] = ((e.flip >> c) & 1u) ? -1.0 * u[c] : u[c];
 }
 
-__global__ void amr_bc_kernel(const AmrBc* t, long long n, AmrBufs B, int k, int N) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const AmrBc e = t[q];
-        double* a = B.p[e.b * 4 + k];
-        const long long S = B.S[e.b];
-        for (int c = 0; c < N; ++c) {
-            const double v = a[c * S + e.sq];
-            a[c * S + e.dq] = ((e.odd >> c) & 1u) ? -1.0 * v : 1.0 * v;
-        }
+__global__ void __launch_bounds__(128) amr_interp_kernel(const AmrInterp* t, long long n, AmrBufs B, int dk, int knew,
+                                                         int kold, int mode, double alpha, double beta, int N, int D, int pc) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
+        amr_interp_cell(t[q], B, dk, knew, kold, mode, alpha, beta, N, D, pc);
+}
+
+// The ghost cells of a level's array k in one launch: same-level copies, coarse-fine interpolation and the
+// physical boundaries (whose cells are images of cells within the domain, resolved when the tables are built). With
+// ctl set also the level's step size and wave-speed accumulator for the stages that follow. As separate
+// launches (copies, interpolation, a boundary launch a direction, the step size) a fill took four to five of
+// about 7 us each, all latency.
+struct AmrFillArgs {
+    const AmrSame* same;
+    const AmrInterp* interp;
+    long long n_same, n_interp;
+    AmrBufs B;
+    int k, knew, kold, mode;
+    double alpha, beta;
+    int N, D, pc;
+    double* dt;  // null: leave the step control alone
+    double dt_value;
+    unsigned long long* cmax;
+};
+
+__global__ void __launch_bounds__(128) amr_fill_kernel(AmrFillArgs a) {
+    if (a.dt && blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.dt = a.dt_value;
+        *a.cmax = 0ull;
+    }
+    // the interpolated cells, which take longest, first
+    const long long total = a.n_interp + a.n_same;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
+        if (q < a.n_interp) amr_interp_cell(a.interp[q], a.B, a.k, a.knew, a.kold, a.mode, a.alpha, a.beta, a.N, a.D, a.pc);
+        else amr_copy_cell(a.same[q - a.n_interp], a.B, a.k, a.N);
     }
 }
 
@@ -326,32 +359,55 @@ struct AmrCfArgs {
     int id_riemann;     // Physics.RiemannSolver
     double dx[3];       // cell sizes of the level computing the fluxes
     int role;           // 0: coarse (CrseInit, scale -w), 1: fine (FineAdd, scale w)
+    int first;          // the registers start from zero (the coarse level's first stage)
 };
 
+// Flux-register contributions of a stage, one thread per face: coarse faces, or the 2^(D-1) fine faces of a
+// register on neighbouring lanes, whose fluxes the first of them adds in order. Two register sets (a middle
+// level's as the coarse and as the fine side) share a launch. It reads the stage's input only, so it runs on
+// a stream of its own beside the stage kernel.
 template <class M, int SCHEME, bool MIX>
-__global__ void amr_cf_kernel(AmrCfArgs A) {
+__device__ __forceinline__ void amr_cf_faces(const AmrCfArgs& A, int item) {
     constexpr int N = M::N, NC = M::NC;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n; t += gridDim.x * blockDim.x) {
+    const int nf = (A.role == 0) ? 1 : (M::D == 3 ? 4 : 2);
+    const int t = item / nf, a = item % nf;
+    const bool on = t < A.n;
+    double F[N], fnc[NC];
+    int d = 0;
+    if (on) {
         const AmrCf& f = A.cf[t];
-        const double dA = (f.d == 0) ? A.dA[0] : (f.d == 1 ? A.dA[1] : A.dA[2]);
-        const double dxd = (f.d == 0) ? A.dx[0] : (f.d == 1 ? A.dx[1] : A.dx[2]);
-        double F[N], fnc[NC];
-        if (A.role == 0) {
-            amr_face_flux<M, SCHEME, MIX>(A.B.p[f.cbox * 4 + A.k], A.grids[f.cbox], f.d, f.cface[0], f.cface[1],
-                                          f.cface[2], A.e, A.id_k, A.code, A.id_riemann, dxd, F, fnc, nullptr);
-            for (int c = 0; c < N; ++c) A.reg[(long long)t * N + c] += (-A.w) * (F[c] * dA);
-            for (int c = 0; c < NC; ++c) A.reg_nc[(long long)t * NC + c] += (-A.w) * (fnc[c] * dA);
-        } else {
-            const int nf = (M::D == 3) ? 4 : 2;
-            for (int a = 0; a < nf; ++a) {
-                amr_face_flux<M, SCHEME, MIX>(A.B.p[f.fbox[a] * 4 + A.k], A.grids[f.fbox[a]], f.d, f.fface[a][0],
-                                              f.fface[a][1], f.fface[a][2], A.e, A.id_k, A.code, A.id_riemann, dxd, F,
-                                              fnc, nullptr);
-                for (int c = 0; c < N; ++c) A.reg[(long long)t * N + c] += A.w * (F[c] * dA);
-                for (int c = 0; c < NC; ++c) A.reg_nc[(long long)t * NC + c] += A.w * (fnc[c] * dA);
-            }
-        }
+        d = f.d;
+        const double dxd = (d == 0) ? A.dx[0] : (d == 1 ? A.dx[1] : A.dx[2]);
+        const int box = (A.role == 0) ? f.cbox : f.fbox[a];
+        const int* face = (A.role == 0) ? f.cface : f.fface[a];
+        amr_face_flux<M, SCHEME, MIX>(A.B.p[box * 4 + A.k], A.grids[box], d, face[0], face[1], face[2], A.e, A.id_k,
+                                      A.code, A.id_riemann, dxd, F, fnc, nullptr);
     }
+    const double dA = (d == 0) ? A.dA[0] : (d == 1 ? A.dA[1] : A.dA[2]);
+    const double w = (A.role == 0) ? -A.w : A.w;
+    auto add = [&](double* reg, double v) {
+        const double x = w * (v * dA);
+        double s = 0.0;
+        if (on && a == 0) s = (A.first ? 0.0 : *reg) + x;
+        for (int h = 1; h < nf; ++h) {
+            const double y = __shfl_down_sync(0xffffffffu, x, h);
+            if (a == 0) s += y;
+        }
+        if (on && a == 0) *reg = s;
+    };
+#pragma unroll
+    for (int c = 0; c < N; ++c) add(A.reg + (long long)(on ? t : 0) * N + c, F[c]);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) add(A.reg_nc + (long long)(on ? t : 0) * NC + c, fnc[c]);
+}
+
+constexpr int kCfThreads = 64;
+
+// blocks [0, blocks0): the first set, the others the second
+template <class M, int SCHEME, bool MIX>
+__global__ void __launch_bounds__(kCfThreads) amr_cf_kernel(AmrCfArgs A0, AmrCfArgs A1, int blocks0) {
+    if ((int)blockIdx.x < blocks0) amr_cf_faces<M, SCHEME, MIX>(A0, blockIdx.x * kCfThreads + threadIdx.x);
+    else amr_cf_faces<M, SCHEME, MIX>(A1, (blockIdx.x - blocks0) * kCfThreads + threadIdx.x);
 }
 
 // FluxRegister::Reflux and RefluxSourceTerms: one thread per coarse cell, its faces in list order.
@@ -442,17 +498,20 @@ __global__ void amr_avg_kernel(const AmrAvg* t, long long n, AmrBufs B, int kc, 
         const AmrAvg& e = t[q];
         double* C = B.p[e.cb * 4 + kc];
         const long long Sc = B.S[e.cb];
-        for (int c = 0; c < N; ++c) {
-            double s = 0.0;
-            for (int h = 0; h < nchild; ++h) s += B.p[e.fb[h] * 4 + kf][c * B.S[e.fb[h]] + e.fq[h]];
-            C[c * Sc + e.cq] = volfrac * s;
+        double s[kAmrMaxComp];
+#pragma unroll
+        for (int c = 0; c < kAmrMaxComp; ++c) s[c] = 0.0;
+        for (int h = 0; h < nchild; ++h) {
+            const double* src = B.p[e.fb[h] * 4 + kf] + e.fq[h];
+            const long long S = B.S[e.fb[h]];
+#pragma unroll
+            for (int c = 0; c < kAmrMaxComp; ++c)
+                if (c < N) s[c] += src[c * S];
         }
+#pragma unroll
+        for (int c = 0; c < kAmrMaxComp; ++c)
+            if (c < N) C[c * Sc + e.cq] = volfrac * s[c];
     }
-}
-
-__global__ void amr_set_kernel(double* dt, double v, unsigned long long* cmax) {
-    *dt = v;
-    if (cmax) *cmax = 0ull;
 }
 
 }  // namespace compas
