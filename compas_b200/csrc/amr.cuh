@@ -215,7 +215,7 @@ template <class M, int SCHEME, bool MIX>
 __device__ void amr_face_flux(const double* U, const Grid& g, int d, int i, int j, int k, const Eos& e, int id_k,
                               int code, int id_riemann, double dxd, double* F, double* fnc, unsigned int* err) {
     using PT = typename std::conditional<MIX, float, double>::type;
-    constexpr int N = M::N, D = M::D;
+    constexpr int N = M::N;
     constexpr bool NPH = (M::KIND == kModelFiveN);
     constexpr bool SXN = (M::KIND == kModelSixN);
     PT P[6][N];

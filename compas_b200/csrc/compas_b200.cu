@@ -54,42 +54,12 @@ static int fail(int code, const std::string& msg) {
 // source/Class_Compressible5Eq_NPhase_PhaseField.cpp:133-205).
 enum { kBcPeriodic = 0, kBcExtrap = 1, kBcEven = 2, kBcOdd = 3 };
 
-__device__ __forceinline__ int bc_kind(int code, int n, int d, int D, int m0) {
-    const bool mom = (n >= m0 && n < m0 + D);
-    switch (code) {
-        case 0: return kBcPeriodic;
-        case 2: return kBcExtrap;
-        case 3:
-        case 4: return (mom && n - m0 == d) ? kBcOdd : kBcEven;
-        default: return mom ? kBcOdd : kBcEven;  // 5: no-slip wall
-    }
-}
-
 struct BcArgs {
     double* U;
     Grid g;
     int N, D, m0;
     int lo[3], hi[3];
 };
-
-// Map one coordinate of a ghost cell to its source along d; returns the sign factor.
-__device__ __forceinline__ double bc_map(int& x, int len, int code_lo, int code_hi, int n, int d, int D, int m0) {
-    if (x < 0) {
-        const int kind = bc_kind(code_lo, n, d, D, m0);
-        if (kind == kBcPeriodic) { x += len; return 1.0; }
-        if (kind == kBcExtrap) { x = 0; return 1.0; }
-        x = -1 - x;
-        return kind == kBcOdd ? -1.0 : 1.0;
-    }
-    if (x >= len) {
-        const int kind = bc_kind(code_hi, n, d, D, m0);
-        if (kind == kBcPeriodic) { x -= len; return 1.0; }
-        if (kind == kBcExtrap) { x = len - 1; return 1.0; }
-        x = 2 * len - 1 - x;
-        return kind == kBcOdd ? -1.0 : 1.0;
-    }
-    return 1.0;
-}
 
 // One thread per ghost cell (all components). Ghost cells are enumerated as the z slabs (full
 // padded planes), then the y slabs of the valid z range, then the x slabs of the valid y, z range.
@@ -100,53 +70,69 @@ __host__ __device__ __forceinline__ long long ghost_count(const Grid& g) {
     return 2LL * g.gz * g.pxy + 2LL * g.ng * g.px * g.n[2] + 2LL * g.ng * g.n[1] * g.n[2];
 }
 
-// Ghost cell (i, j, k) of U from the valid cell its coordinates map to, all components.
+// Ghost cell (i, j, k) of U from the valid cell its coordinates map to (ghost_source), all components: loaded
+// together and then stored, so that a cell costs one memory latency and not one per component.
+constexpr int kMaxComp = 16;
 __device__ __forceinline__ void fill_cell(double* U, const Grid& g, int N, int D, int m0, const int* lo,
                                           const int* hi, int i, int j, int k) {
-    const long long dst = g.at(i, j, k);
-    for (int n = 0; n < N; ++n) {
-        int si = i, sj = j, sk = k;
-        double sgn = bc_map(si, g.n[0], lo[0], hi[0], n, 0, D, m0);
-        sgn *= bc_map(sj, g.n[1], lo[1], hi[1], n, 1, D, m0);
-        if (D == 3) sgn *= bc_map(sk, g.n[2], lo[2], hi[2], n, 2, D, m0);
-        U[n * g.S + dst] = sgn * U[n * g.S + g.at(si, sj, sk)];
-    }
+    unsigned odd = 0;
+    const int si = ghost_source(i, g.n[0], lo[0], hi[0], 0, odd);
+    const int sj = ghost_source(j, g.n[1], lo[1], hi[1], 1, odd);
+    const int sk = (D == 3) ? ghost_source(k, g.n[2], lo[2], hi[2], 2, odd) : k;
+    const double* src = U + g.at(si, sj, sk);
+    double* dst = U + g.at(i, j, k);
+    odd = (odd & ((1u << D) - 1u)) << m0;  // as a mask of components
+    double v[kMaxComp];
+#pragma unroll
+    for (int n = 0; n < kMaxComp; ++n)
+        if (n < N) v[n] = src[n * g.S];
+#pragma unroll
+    for (int n = 0; n < kMaxComp; ++n)
+        if (n < N) dst[n * g.S] = ((odd >> n) & 1u) ? -v[n] : v[n];
 }
 
-// Fill ghost cell number q (enumeration above) of U, all components.
+// Ghost cell number q (enumeration above) of U, all components. I: the index type, 32 bits where the count
+// allows (the divisions by the row and plane sizes are the kernel's arithmetic).
+template <class I>
+__device__ __forceinline__ void fill_ghost_cell_t(double* U, const Grid& g, int N, int D, int m0, const int* lo,
+                                                  const int* hi, I q) {
+    const I PX = (I)g.px, PY = (I)(g.n[1] + 2 * g.ng);
+    const I nz_slab = 2 * (I)g.gz * PX * PY;
+    const I ny_slab = 2 * (I)g.ng * PX * (I)g.n[2];
+    int i, j, k;
+    if (q < nz_slab) {
+        const I plane = PX * PY;
+        const int s = (int)(q / plane);
+        const I r = q - (I)s * plane;
+        const I row = r / PX;
+        i = (int)(r - row * PX) - g.ng;
+        j = (int)row - g.ng;
+        k = (s < g.gz) ? s - g.gz : g.n[2] + (s - g.gz);
+    } else if (q < nz_slab + ny_slab) {
+        const I r0 = q - nz_slab;
+        const I plane = PX * (I)g.n[2];
+        const int s = (int)(r0 / plane);
+        const I r = r0 - (I)s * plane;
+        const I row = r / PX;
+        i = (int)(r - row * PX) - g.ng;
+        k = (int)row;
+        j = (s < g.ng) ? s - g.ng : g.n[1] + (s - g.ng);
+    } else {
+        const I r0 = q - nz_slab - ny_slab;
+        const I col = (I)g.n[1] * (I)g.n[2];
+        const int s = (int)(r0 / col);
+        const I r = r0 - (I)s * col;
+        k = (int)(r / (I)g.n[1]);
+        j = (int)(r - (I)k * (I)g.n[1]);
+        i = (s < g.ng) ? s - g.ng : g.n[0] + (s - g.ng);
+    }
+    fill_cell(U, g, N, D, m0, lo, hi, i, j, k);
+}
+
 __device__ __forceinline__ void fill_ghost_cell(double* U, const Grid& g, int N, int D, int m0, const int* lo,
                                                 const int* hi, long long q) {
-    const long long PX = g.px, PY = g.pxy / g.px;
-    const long long nz_slab = 2LL * g.gz * PX * PY;
-    const long long ny_slab = 2LL * g.ng * PX * g.n[2];
-    {
-        int i, j, k;
-        if (q < nz_slab) {
-            const long long plane = PX * PY;
-            const int s = (int)(q / plane);
-            const long long r = q % plane;
-            i = (int)(r % PX) - g.ng;
-            j = (int)(r / PX) - g.ng;
-            k = (s < g.gz) ? s - g.gz : g.n[2] + (s - g.gz);
-        } else if (q < nz_slab + ny_slab) {
-            const long long r0 = q - nz_slab;
-            const long long row = PX * g.n[2];
-            const int s = (int)(r0 / row);
-            const long long r = r0 % row;
-            i = (int)(r % PX) - g.ng;
-            k = (int)(r / PX);
-            j = (s < g.ng) ? s - g.ng : g.n[1] + (s - g.ng);
-        } else {
-            const long long r0 = q - nz_slab - ny_slab;
-            const long long col = (long long)g.n[1] * g.n[2];
-            const int s = (int)(r0 / col);
-            const long long r = r0 % col;
-            j = (int)(r % g.n[1]);
-            k = (int)(r / g.n[1]);
-            i = (s < g.ng) ? s - g.ng : g.n[0] + (s - g.ng);
-        }
-        fill_cell(U, g, N, D, m0, lo, hi, i, j, k);
-    }
+    if (ghost_count(g) < (1LL << 31)) fill_ghost_cell_t<unsigned>(U, g, N, D, m0, lo, hi, (unsigned)q);
+    else fill_ghost_cell_t<long long>(U, g, N, D, m0, lo, hi, q);
 }
 
 __global__ void fill_boundary_kernel(BcArgs a) {
@@ -609,8 +595,8 @@ static int tune_candidates(F&& launch, cudaStream_t st, int reps, TuneChoice* be
     return rc;
 }
 
-// The launch shape of a box that nothing has tuned: a box of fewer tiles than the GPU has SMs takes the shape
-// with one large CTA per tile (a 64^2 FIVEEQS WENO5 FP64 stage, 16 tiles: shape 0 / 1 see kern_impl.cuh).
+// The launch shape of a box that nothing has tuned: a box of fewer tiles than the GPU has SMs is bound by one
+// tile's time and takes shape 1 (kern_impl.cuh: in 3D one large CTA per tile, in 2D smaller tiles).
 static int default_shape(const compas_b200_parm* p, const compas_b200_geom* g) {
     const int ts = (p->dim == 2) ? kTile2 : kTile3;
     const long long tiles = (long long)((g->n[0] + ts - 1) / ts) * ((g->n[1] + ts - 1) / ts) *
@@ -2053,6 +2039,8 @@ int compas_b200_level_step_host(compas_b200_level* lv, const double* host_in, do
     a.cmax = &lv->ctl->cmax;
     a.err = &lv->ctl->err;
     a.order = 0;
+    // the slabs are layers of kTile2 / kTile3 cells, which shape 1 of the 2D kernels does not use
+    const int shape = (D == 2 && lv->shape == 1) ? 0 : lv->shape;
     double* bufs_in[3] = {lv->U, lv->U1, lv->U2};
     double* bufs_out[3] = {lv->U1, lv->U2, lv->U};
     int rc;
@@ -2070,7 +2058,7 @@ int compas_b200_level_step_host(compas_b200_level* lv, const double* host_in, do
             a.Uout = bufs_out[s];
             a.tile_base = L0[c] * layer_tiles;
             a.tile_count = (L0[c + 1] - L0[c]) * layer_tiles;
-            if ((rc = launch_stage(p, a, st, 0, lv->shape, lv->use_tma ? &lv->maps[s] : nullptr))) return rc;
+            if ((rc = launch_stage(p, a, st, 0, shape, lv->use_tma ? &lv->maps[s] : nullptr))) return rc;
             if (s < 2) {
                 if ((rc = fill(bufs_out[s], c))) return rc;
             } else {

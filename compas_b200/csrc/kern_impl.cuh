@@ -38,12 +38,16 @@ template <bool MIX> struct ShapeParams<true, 2, MIX, 0> { static constexpr int N
 template <bool MIX> struct ShapeParams<true, 2, MIX, 1> { static constexpr int NT = 272, MINB = 1; };
 template <bool MIX> struct ShapeParams<true, 2, MIX, 2> { static constexpr int NT = 136, MINB = 4; };
 
-template <class M, bool FACES, bool MIX, int S>
+// In 2D, shape 1 of the single-box kernel takes 8^2 tiles: a box of few tiles is bound by the time of one
+// tile, and four small ones on four SMs take a fraction of it (more halo, 2.5 conversions a cell for 1.75, so
+// not where the larger tiles fill the GPU). LIST: the box-list kernel, whose tile counts are those of 16^2.
+template <class M, bool FACES, bool MIX, int S, bool LIST = false>
 struct LaunchShape {
-    static constexpr int TS = (M::D == 2) ? kTile2 : kTile3;
+    static constexpr bool SMALL = (M::D == 2 && !FACES && !LIST && S == 1);
+    static constexpr int TS = SMALL ? kTile2 / 2 : (M::D == 2) ? kTile2 : kTile3;
     static constexpr int TZ = (M::D == 2) ? 1 : TS;
-    static constexpr int NT = ShapeParams<FACES, M::D, MIX, S>::NT;
-    static constexpr int MINB = ShapeParams<FACES, M::D, MIX, S>::MINB;
+    static constexpr int NT = SMALL ? 192 : ShapeParams<FACES, M::D, MIX, S>::NT;
+    static constexpr int MINB = SMALL ? 2 : ShapeParams<FACES, M::D, MIX, S>::MINB;
 };
 
 // One CTA per tile of the box.
@@ -132,7 +136,7 @@ static cudaError_t launch_stage_m(const KernelChoice& k, const StageArgs& a, cud
 // Persistent box-list launch: one resident wave of CTAs walks the tiles of every box.
 template <class M, int SCHEME, bool MIX, int SH>
 static cudaError_t launch_list_v(const ListArgs& L, cudaStream_t st) {
-    using S = LaunchShape<M, SCHEME == 2, MIX, SH>;
+    using S = LaunchShape<M, SCHEME == 2, MIX, SH, true>;
     constexpr size_t SMEM = tile_smem<M, SCHEME, MIX, kVarPlain, S::TS, S::TZ, S::MINB>();
     auto kern = stage_list_kernel<M, SCHEME, MIX, S::TS, S::TS, S::TZ, S::NT, S::MINB>;
     static int grid = 0;

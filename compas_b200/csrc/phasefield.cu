@@ -929,6 +929,202 @@ __global__ void __launch_bounds__(kBlockThreads) k_mg_vcycle_block(const MgLevel
     for (int q = threadIdx.x; q < (int)levels[l0].m.nv; q += blockDim.x) levels[l0].x[q] = sl[l0].x[q];
 }
 
+// ---- the single-block cycle of 2D levels with even, two-colourable rows ---------------------------------
+// The same cycle with less latency per step (the single block is all that runs meanwhile): arrays in
+// shared memory by offset (k_mg_vcycle_block reaches them through generic pointers kept in shared memory), face
+// coefficients already divided by h^2 and zero on the walls, so that a neighbour sum has no branch, a cell's
+// constants held in registers over the passes of a smoothing, the residual formed and restricted in one
+// step, and 1/idiag formed once instead of a division per cell and residual. Bound by the latency of some 90
+// dependent steps. B200, levels 64 x 32 .. 4 x 2 (a 512 x 256 solve): @@ us, 87 us as k_mg_vcycle_block.
+struct Blk2 {
+    int n0, n1, hw, ncol, nv;
+    bool p0, p1;
+    double *x, *b, *id, *dg, *fx, *fy;  // fx[(n0 + 1) n1], fy[n0 (n1 + 1)]
+    __device__ __forceinline__ double off(int i, int j) const {
+        const int q = i + n0 * j;
+        const int w = (i > 0) ? q - 1 : (p0 ? q + n0 - 1 : q), e = (i < n0 - 1) ? q + 1 : (p0 ? q - n0 + 1 : q);
+        const int s = (j > 0) ? q - n0 : (p1 ? q + n0 * (n1 - 1) : q), n = (j < n1 - 1) ? q + n0 : (p1 ? q - n0 * (n1 - 1) : q);
+        const double* f = fx + i + (n0 + 1) * j;
+        double o = f[0] * x[w];
+        o += f[1] * x[e];
+        o += fy[q] * x[s];
+        o += fy[q + n0] * x[n];
+        return o;
+    }
+};
+
+template <class T>
+__device__ __forceinline__ void blk2_smooth(const Blk2& L, int sweeps, bool reverse) {
+    if (L.ncol <= T::size()) {
+        // a thread owns one cell of each colour and keeps its constants
+        const int t = T::id();
+        const bool on = t < L.ncol;
+        const int j = on ? t / L.hw : 0, ih = on ? 2 * (t - j * L.hw) : 0;
+        int q[2], nb[2][4];
+        double c[2][4], b[2], id[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = ih + ((j + k) & 1);
+            q[k] = i + L.n0 * j;
+            nb[k][0] = (i > 0) ? q[k] - 1 : (L.p0 ? q[k] + L.n0 - 1 : q[k]);
+            nb[k][1] = (i < L.n0 - 1) ? q[k] + 1 : (L.p0 ? q[k] - L.n0 + 1 : q[k]);
+            nb[k][2] = (j > 0) ? q[k] - L.n0 : (L.p1 ? q[k] + L.n0 * (L.n1 - 1) : q[k]);
+            nb[k][3] = (j < L.n1 - 1) ? q[k] + L.n0 : (L.p1 ? q[k] - L.n0 * (L.n1 - 1) : q[k]);
+            c[k][0] = L.fx[i + (L.n0 + 1) * j];
+            c[k][1] = L.fx[i + 1 + (L.n0 + 1) * j];
+            c[k][2] = L.fy[q[k]];
+            c[k][3] = L.fy[q[k] + L.n0];
+            b[k] = L.b[q[k]];
+            id[k] = L.id[q[k]];
+        }
+        for (int s = 0; s < sweeps; ++s) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool one = (u == 1) != reverse;  // colour 1's turn
+                const int k0 = one ? q[1] : q[0];
+                double o = (one ? c[1][0] : c[0][0]) * L.x[one ? nb[1][0] : nb[0][0]];
+                o += (one ? c[1][1] : c[0][1]) * L.x[one ? nb[1][1] : nb[0][1]];
+                o += (one ? c[1][2] : c[0][2]) * L.x[one ? nb[1][2] : nb[0][2]];
+                o += (one ? c[1][3] : c[0][3]) * L.x[one ? nb[1][3] : nb[0][3]];
+                if (on) L.x[k0] = ((one ? b[1] : b[0]) + o) * (one ? id[1] : id[0]);
+                T::sync();
+            }
+        }
+        return;
+    }
+    for (int s = 0; s < sweeps; ++s)
+        for (int u = 0; u < 2; ++u) {
+            const int color = reverse ? 1 - u : u;
+            for (int t = T::id(); t < L.ncol; t += T::size()) {
+                const int j = t / L.hw, i = 2 * (t - j * L.hw) + ((j + color) & 1), q = i + L.n0 * j;
+                L.x[q] = (L.b[q] + L.off(i, j)) * L.id[q];
+            }
+            T::sync();
+        }
+}
+
+template <class T>
+__device__ __forceinline__ void blk2_down(const Blk2& L, const Blk2& C) {
+    blk2_smooth<T>(L, 2, false);
+    for (int q = T::id(); q < C.nv; q += T::size()) {
+        const int J = q / C.n0, I = q - J * C.n0;
+        double sum = 0.0;
+#pragma unroll
+        for (int dj = 0; dj < 2; ++dj)
+#pragma unroll
+            for (int di = 0; di < 2; ++di) {
+                const int i = 2 * I + di, j = 2 * J + dj, f = i + L.n0 * j;
+                sum += L.b[f] - (L.x[f] * L.dg[f] - L.off(i, j));
+            }
+        C.b[q] = 0.25 * sum;
+        C.x[q] = 0.0;
+    }
+    T::sync();
+}
+
+template <class T>
+__device__ __forceinline__ void blk2_up(const Blk2& L, const Blk2& C) {
+    for (int t = T::id(); t < L.nv / 2; t += T::size()) {  // two cells of one parent
+        const int j = t / L.hw, I = t - j * L.hw, q = 2 * I + L.n0 * j;
+        const double c = C.x[I + C.n0 * (j >> 1)];
+        L.x[q] += c;
+        L.x[q + 1] += c;
+    }
+    T::sync();
+    blk2_smooth<T>(L, 2, true);
+}
+
+constexpr int kBlk2Levels = 8;
+
+// x_zero: the first level's x starts from zero (and is not read)
+__global__ void __launch_bounds__(kBlockThreads) k_mg_vcycle_block_2d(const MgLevel* levels, int l0, int nl, int x_zero) {
+    extern __shared__ double bsm[];
+    __shared__ Blk2 sl[kBlk2Levels];
+    __shared__ MgLevel gl[kBlk2Levels];
+    __shared__ int first[kBlk2Levels + 1];  // first cell of each level among all
+    const int nlv = nl - l0;
+    for (int w = threadIdx.x; w < nlv * (int)(sizeof(MgLevel) / 8); w += blockDim.x)
+        reinterpret_cast<unsigned long long*>(gl)[w] = reinterpret_cast<const unsigned long long*>(levels + l0)[w];
+    __syncthreads();
+    if (threadIdx.x < nlv) {
+        long long o = 0;
+        int cells = 0;
+        for (int l = 0; l < (int)threadIdx.x; ++l) {
+            o += block_cycle_doubles(gl[l].m);
+            cells += (int)gl[l].m.nv;
+        }
+        const PfDims& m = gl[threadIdx.x].m;
+        Blk2 L;
+        L.n0 = m.n[0];
+        L.n1 = m.n[1];
+        L.hw = L.n0 / 2;
+        L.nv = L.n0 * L.n1;
+        L.ncol = L.nv / 2;
+        L.p0 = m.periodic[0];
+        L.p1 = m.periodic[1];
+        L.x = bsm + o;
+        L.b = L.x + L.nv;
+        L.id = L.b + L.nv;
+        L.dg = L.id + L.nv;
+        L.fx = L.dg + L.nv;
+        L.fy = L.fx + (L.n0 + 1) * L.n1;
+        sl[threadIdx.x] = L;
+        first[threadIdx.x] = cells;
+        if ((int)threadIdx.x == nlv - 1) first[nlv] = cells + L.nv;
+    }
+    __syncthreads();
+    // every level's constants in one loop over all cells: a cell brings its low x and y faces, the last of a row or
+    // column the high one too (all loads of a round in flight together)
+    for (int u = threadIdx.x; u < first[nlv]; u += blockDim.x) {
+        int l = 0;
+        while (u >= first[l + 1]) ++l;
+        const MgLevel& G = gl[l];
+        const Blk2 L = sl[l];
+        const int q = u - first[l], j = q / L.n0, i = q - j * L.n0, fq = i + (L.n0 + 1) * j;
+        const bool ex = (i == L.n0 - 1), ey = (j == L.n1 - 1);
+        const double id = G.idiag[q], bx = G.beta[0][fq], by = G.beta[1][q];
+        const double bxe = ex ? G.beta[0][fq + 1] : 0.0, bye = ey ? G.beta[1][q + L.n0] : 0.0;
+        double x = 0.0, b = 0.0;
+        if (l == 0) {
+            if (!x_zero) x = G.x[q];
+            b = G.b[q];
+        }
+        L.id[q] = id;
+        L.dg[q] = 1.0 / id;
+        L.fx[fq] = (!L.p0 && i == 0) ? 0.0 : bx * G.ih2[0];
+        L.fy[q] = (!L.p1 && j == 0) ? 0.0 : by * G.ih2[1];
+        if (ex) L.fx[fq + 1] = L.p0 ? bxe * G.ih2[0] : 0.0;
+        if (ey) L.fy[q + L.n0] = L.p1 ? bye * G.ih2[1] : 0.0;
+        if (l == 0) {
+            L.x[q] = x;
+            L.b[q] = b;
+        }
+    }
+    __syncthreads();
+    // levels lw .. nlv-1, those a warp covers with a cell of each colour a lane, run on the first warp alone
+    int lw = nlv;
+    while (lw > 0 && sl[lw - 1].ncol <= 32) --lw;
+    const int lb = (lw < nlv - 1) ? lw : nlv - 1;  // the block's downward steps are 0 .. lb-1
+    for (int l = 0; l < lb; ++l) blk2_down<BlockTeam>(sl[l], sl[l + 1]);
+    if (lw == nlv) {
+        for (int s = 0; s < 8; ++s) {
+            blk2_smooth<BlockTeam>(sl[nlv - 1], 1, false);
+            blk2_smooth<BlockTeam>(sl[nlv - 1], 1, true);
+        }
+    } else if (threadIdx.x < 32) {
+        for (int l = lw; l < nlv - 1; ++l) blk2_down<WarpTeam>(sl[l], sl[l + 1]);
+        for (int s = 0; s < 8; ++s) {
+            blk2_smooth<WarpTeam>(sl[nlv - 1], 1, false);
+            blk2_smooth<WarpTeam>(sl[nlv - 1], 1, true);
+        }
+        for (int l = nlv - 2; l >= lw; --l) blk2_up<WarpTeam>(sl[l], sl[l + 1]);
+    }
+    __syncthreads();
+    for (int l = lb - 1; l >= 0; --l) blk2_up<BlockTeam>(sl[l], sl[l + 1]);
+    const Blk2 L = sl[0];
+    for (int q = threadIdx.x; q < L.nv; q += blockDim.x) levels[l0].x[q] = L.x[q];
+}
+
 // conjugate-gradient scalars kept on the device: cg[0] rz, [1] pAp, [2] alpha, [3] rz_new, [4] beta,
 // [5] the sum of the preconditioned vector (its mean is removed)
 enum CgOp { kCgRz0 = 0, kCgPAp = 1, kCgZsum = 2, kCgRz = 3 };
@@ -1148,13 +1344,21 @@ cudaError_t vcycle(PfLevel* pf, int l, cudaStream_t st, bool x_zero) {
         }
     };
     if (l == pf->mg_block0) {
+        const int nl = (int)pf->mg.size();
+        bool two = (nl - l <= kBlk2Levels);  // every level 2D, two-colourable, with even rows
+        for (int k = l; k < nl; ++k) two = two && pf->mg[k].m.D == 2 && pf->mg[k].rb && pf->mg[k].m.n[0] % 2 == 0;
         static bool attr = false;
         if (!attr) {
             cudaFuncSetAttribute(k_mg_vcycle_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmemMax);
+            cudaFuncSetAttribute(k_mg_vcycle_block_2d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmemMax);
             attr = true;
         }
+        if (two) {
+            k_mg_vcycle_block_2d<<<1, kBlockThreads, pf->mg_block_smem, st>>>(pf->mg_dev, l, nl, x_zero);
+            return cudaGetLastError();
+        }
         if (x_zero) k_zero<<<nb, kThreads, 0, st>>>(L.x, L.m.nv);
-        k_mg_vcycle_block<<<1, kBlockThreads, pf->mg_block_smem, st>>>(pf->mg_dev, l, (int)pf->mg.size());
+        k_mg_vcycle_block<<<1, kBlockThreads, pf->mg_block_smem, st>>>(pf->mg_dev, l, nl);
         return cudaGetLastError();
     }
     if (l + 1 == (int)pf->mg.size()) {

@@ -838,19 +838,27 @@ __device__ __forceinline__ double approx_sqrt(double x) {
     return (x > 0.0) ? r : x;
 }
 
-// Weights of the right face (wp) and the left face (wm) of the centre cell. Where the three indicators lie
-// within 2^+-240 (or all vanish, which the ratio form treats as all equal) the quotients are formed without
-// branches: three reciprocals serve the six ratios, and a face's first denominator, scaled by the squared
-// ratios, gives the reciprocals of the other two (exact relations, so only the last bits need correcting).
-// Other cells, at the edge of a uniform region above all, divide as the reference writes it. Both give
-// the correctly rounded quotients.
+// Weights of the right face (wp) and the left face (wm) of the centre cell. Where the indicators lie within
+// 2^+-240 the quotients are formed without branches: three reciprocals serve the six ratios, and a face's first
+// denominator, scaled by the squared ratios, gives the reciprocals of the other two (exact relations, so only
+// the last bits need correcting). Indicators of 0 (uniform regions and their edges, common in initial states)
+// give the stencils that have them their linear weights' shares and the others none, whatever the others'
+// values: they run as indicators of 1 against 2^200, whose terms round away, with the other weights set to 0.
+// What is left (tiny, infinite or NaN indicators) divides as the reference writes it. All give the
+// correctly rounded quotients.
 __device__ __forceinline__ void weno5_weights(double f_mm, double f_m, double f_c, double f_p, double f_pp, double wp[3],
                                               double wm[3]) {
     const double a = f_p - f_c, b = f_pp - f_p, c = f_c - f_m, g = f_m - f_mm;
-    double IS0 = ((10.0 / 3.0) * a) * a - ((11.0 / 3.0) * a) * b + ((4.0 / 3.0) * b) * b;
-    double IS1 = (-(5.0 / 3.0) * c) * a + ((4.0 / 3.0) * c) * c + ((4.0 / 3.0) * a) * a;
-    double IS2 = ((10.0 / 3.0) * c) * c - ((11.0 / 3.0) * g) * c + ((4.0 / 3.0) * g) * g;
-    if (IS0 == 0.0 && IS1 == 0.0 && IS2 == 0.0) IS0 = IS1 = IS2 = 1.0;
+    const double J0 = ((10.0 / 3.0) * a) * a - ((11.0 / 3.0) * a) * b + ((4.0 / 3.0) * b) * b;
+    const double J1 = (-(5.0 / 3.0) * c) * a + ((4.0 / 3.0) * c) * c + ((4.0 / 3.0) * a) * a;
+    const double J2 = ((10.0 / 3.0) * c) * c - ((11.0 / 3.0) * g) * c + ((4.0 / 3.0) * g) * g;
+    double IS0 = J0, IS1 = J1, IS2 = J2;
+    const bool z0 = (J0 == 0.0), z1 = (J1 == 0.0), z2 = (J2 == 0.0), zero = z0 || z1 || z2;
+    if (zero) {
+        IS0 = z0 ? 1.0 : (J0 < 0x1p240 ? 0x1p200 : J0);
+        IS1 = z1 ? 1.0 : (J1 < 0x1p240 ? 0x1p200 : J1);
+        IS2 = z2 ? 1.0 : (J2 < 0x1p240 ? 0x1p200 : J2);
+    }
     const unsigned h0 = (unsigned)__double2hiint(IS0), h1 = (unsigned)__double2hiint(IS1),
                    h2 = (unsigned)__double2hiint(IS2);
     constexpr unsigned LO = (1023u - 240u) << 20, HI = (1023u + 240u) << 20;
@@ -872,13 +880,18 @@ __device__ __forceinline__ void weno5_weights(double f_mm, double f_m, double f_
             w[1] = div_rn(d1, D1, r1);
             w[2] = div_rn(d2, D2, r2);
         }
+        if (zero) {
+            if (!z0) wp[0] = wm[0] = 0.0;
+            if (!z1) wp[1] = wm[1] = 0.0;
+            if (!z2) wp[2] = wm[2] = 0.0;
+        }
         return;
     }
-    double IS01 = IS0 / IS1;
+    double IS01 = J0 / J1;
     if (isnan(IS01)) IS01 = 1.0;
-    double IS02 = IS0 / IS2;
+    double IS02 = J0 / J2;
     if (isnan(IS02)) IS02 = 1.0;
-    double IS12 = IS1 / IS2;
+    double IS12 = J1 / J2;
     if (isnan(IS12)) IS12 = 1.0;
     const double IS10 = 1.0 / IS01, IS20 = 1.0 / IS02, IS21 = 1.0 / IS12;
     const double s01 = IS01 * IS01, s02 = IS02 * IS02, s10 = IS10 * IS10, s12 = IS12 * IS12, s20 = IS20 * IS20,
