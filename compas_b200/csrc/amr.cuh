@@ -77,6 +77,7 @@ struct AmrLevelH {
     BoxDesc* d_desc[2] = {nullptr, nullptr};
     int* d_nbox = nullptr;
     int* d_tile_off = nullptr;
+    long long tiles = 0;  // tiles of all boxes
     // step control of the level on the device
     double* d_dt = nullptr;
     unsigned long long* d_cmax = nullptr;
@@ -313,8 +314,8 @@ __device__ void amr_face_flux(const double* U, const Grid& g, int d, int i, int 
         } else {
 #pragma unroll
             for (int n = NB0; n < NB1; ++n) {
-                wL[n] = weno5_f32(P[0][n], P[1][n], P[2][n], P[3][n], P[4][n], 1);
-                wR[n] = weno5_f32(P[1][n], P[2][n], P[3][n], P[4][n], P[5][n], -1);
+                wL[n] = weno5_mixed<M::KIND>(P[0][n], P[1][n], P[2][n], P[3][n], P[4][n], 1);
+                wR[n] = weno5_mixed<M::KIND>(P[1][n], P[2][n], P[3][n], P[4][n], P[5][n], -1);
             }
         }
         if constexpr (NPH) {

@@ -595,13 +595,21 @@ static int tune_candidates(F&& launch, cudaStream_t st, int reps, TuneChoice* be
     return rc;
 }
 
-// The launch shape of a box that nothing has tuned: a box of fewer tiles than the GPU has SMs is bound by one
-// tile's time and takes shape 1 (kern_impl.cuh: in 3D one large CTA per tile, in 2D smaller tiles).
+// The launch shape where nothing has tuned it, from the number of 16^2 or 8^3 tiles (kern_impl.cuh). Few tiles
+// are bound by one tile's time, so it goes to shapes with more threads a tile: up to one per SM (148) shape 1
+// (3D: one large CTA a tile; 2D FP64: 8^2 tiles; 32^3 SIXEQS 139 -> 92 us FP64, 51 -> 44 mixed, 128^2 FIVEEQS FP64 66
+// -> 49 us, with launches); 2D mixed up to a wave of shape 0 (592) shape 2 (512 x 256: 54 -> 44 us, 192 x 128: 37 -> 28,
+// shape 1 35).
+static int default_shape(const compas_b200_parm* p, long long tiles) {
+    if (p->id_limiter < 5 || p->thinc) return 0;
+    if (p->dim == 2 && p->precision == 1) return tiles <= 592 ? 2 : 0;
+    return tiles <= 148 ? 1 : 0;
+}
+
 static int default_shape(const compas_b200_parm* p, const compas_b200_geom* g) {
     const int ts = (p->dim == 2) ? kTile2 : kTile3;
-    const long long tiles = (long long)((g->n[0] + ts - 1) / ts) * ((g->n[1] + ts - 1) / ts) *
-                            (p->dim == 3 ? (g->n[2] + ts - 1) / ts : 1);
-    return (p->id_limiter >= 5 && !p->thinc && tiles <= 148) ? 1 : 0;
+    return default_shape(p, (long long)((g->n[0] + ts - 1) / ts) * ((g->n[1] + ts - 1) / ts) *
+                                (p->dim == 3 ? (g->n[2] + ts - 1) / ts : 1));
 }
 
 // The tuned launch shape / tile order of a single box of this size, if a level has tuned it in this

@@ -13,18 +13,20 @@ namespace compas {
 // Launch shapes of the stage kernels (threads per CTA, CTAs per SM) among which the autotuner picks;
 // the tile is 8^3 in 3D and 16^2 in 2D for every shape. The register budget is set per SM
 // sub-partition (16384 registers each, warps dealt round-robin). Shape 0 is the default where nothing is
-// tuned, shape 1 that of boxes of fewer tiles than SMs (default_shape in compas_b200.cu).
+// tuned and the tiles fill the GPU; default_shape (compas_b200.cu) has the rule for fewer.
 //
 // stage_tile (FACES = false): its passes have 512 (3D) or 18 x 16 x components (2D) reconstruction items and
-// 576 or 272 faces, so 288 threads fill both nearly evenly. B200, us per stage, shapes 0 / 1 / 2:
-// 96^3 SIXEQS WENO5 mixed 250 / 266 / 285, FP64 793 / 810 / 888; 1024 x 512 FIVEEQS WENO5B mixed
-// 87 / 125 / 95, FP64 260 / 324 / 298; 128^2 FIVEEQS WENO5 FP64 (64 tiles) 68 / 58 / 82.
+// 576 or 272 faces, so 288 threads fill both nearly evenly; in 3D mixed, 320 (ten warps, the most that the
+// registers of 288 leave room for) do better for being more warps. B200, us per stage: 128^3 SIXEQS WENO5
+// mixed with 192 / 256 / 288 / 320 threads x 2 (TMA halos) 570 / 518 / 546 / 513, WENO5B 288 / 320 627 / 586;
+// 96^3 FP64 288 x 2 / 576 x 1 / 384 x 1 764 / 810 / 888; 1024 x 512 FIVEEQS WENO5B mixed 144 x 4 / 192 x 3 /
+// 288 x 2 87 / 93 / 95, FP64 288 x 2 / 192 x 3 / 144 x 4 254 / 276 / 298.
 // stage_tile_faces (FACES = true): 576 (3D) or 272 (2D) faces a direction and one thread each.
 template <bool FACES, int D, bool MIX, int S>
 struct ShapeParams;
-template <bool MIX> struct ShapeParams<false, 3, MIX, 0> { static constexpr int NT = 288, MINB = 2; };
+template <bool MIX> struct ShapeParams<false, 3, MIX, 0> { static constexpr int NT = MIX ? 320 : 288, MINB = 2; };
 template <bool MIX> struct ShapeParams<false, 3, MIX, 1> { static constexpr int NT = 576, MINB = 1; };
-template <> struct ShapeParams<false, 3, true, 2> { static constexpr int NT = 192, MINB = 2; };
+template <> struct ShapeParams<false, 3, true, 2> { static constexpr int NT = 256, MINB = 2; };
 template <> struct ShapeParams<false, 3, false, 2> { static constexpr int NT = 384, MINB = 1; };
 template <> struct ShapeParams<false, 2, true, 0> { static constexpr int NT = 144, MINB = 4; };
 template <> struct ShapeParams<false, 2, true, 2> { static constexpr int NT = 288, MINB = 2; };

@@ -827,7 +827,7 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-// sqrt(x), x >= 0, within about one unit in the last place (mixed form): two Newton steps
+// sqrt(x) within about one unit in the last place (mixed form; NaN for x < 0): two Newton steps
 // y (3 - x y^2)/2 on the hardware's estimate of 1/sqrt(x), then x y with its residual folded in.
 __device__ __forceinline__ double approx_sqrt(double x) {
     double y;
@@ -835,7 +835,7 @@ __device__ __forceinline__ double approx_sqrt(double x) {
     y = y * fma(-0.5 * x, y * y, 1.5);
     const double s = x * y;
     const double r = fma(fma(-s, s, x), 0.5 * y, s);
-    return (x > 0.0) ? r : x;
+    return (x > 0.0) ? r : ((x < 0.0) ? __longlong_as_double(0x7ff8000000000000ll) : x);
 }
 
 // Weights of the right face (wp) and the left face (wm) of the centre cell. Where the indicators lie within
@@ -1101,9 +1101,58 @@ __device__ __forceinline__ void weno5_both_f32(float f_mm, float f_m, float f_c,
     vm = f_c + weno5_corr_f32(g, c, a, b, -1, wm);
 }
 
-__device__ __forceinline__ float weno5_f32(float f_mm, float f_m, float f_c, float f_p, float f_pp, int side) {
+// The N-phase model's FP32 weights: the same ratio form with the reference's coefficients as they stand and
+// the vanishing indicators told apart by comparisons. Its flows (sharp interfaces under a limiter that
+// switches on slope sums of 1e-10) carry a change of rounding in these weights to 5e-6 of the state within 20
+// small-grid steps, so they keep the rounding they have had; the two faces share indicators and ratios.
+__device__ __forceinline__ void weno5_both_f32_nphase(float f_mm, float f_m, float f_c, float f_p, float f_pp, float& vp,
+                                                      float& vm) {
+    const float a = f_p - f_c, b = f_pp - f_p, c = f_c - f_m, g = f_m - f_mm;
+    const float IS0 = __fmaf_rn((10.0f / 3.0f) * a, a, __fmaf_rn(-(11.0f / 3.0f) * a, b, (4.0f / 3.0f) * b * b));
+    const float IS1 = __fmaf_rn(-(5.0f / 3.0f) * c, a, (4.0f / 3.0f) * __fmaf_rn(c, c, a * a));
+    const float IS2 = __fmaf_rn((10.0f / 3.0f) * c, c, __fmaf_rn(-(11.0f / 3.0f) * g, c, (4.0f / 3.0f) * g * g));
+    const bool z0 = (IS0 == 0.0f), z1 = (IS1 == 0.0f), z2 = (IS2 == 0.0f);
+    const bool anyz = z0 | z1 | z2;
+    // |ratio|: an indicator can round slightly below zero; the clamp then also bounds the square
+    const float r01 = fminf(fabsf(IS0 * __fdividef(1.0f, IS1)), 1.0e18f);
+    const float r02 = fminf(fabsf(IS0 * __fdividef(1.0f, IS2)), 1.0e18f);
+    const float s01 = anyz ? 0.0f : r01 * r01, s02 = anyz ? 0.0f : r02 * r02;
+    const float d1 = 0.6f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float d0 = k ? 0.1f : 0.3f, d2 = k ? 0.3f : 0.1f;
+        float e0, e1, e2;
+        if (k == 0) {
+            e0 = __fmaf_rn(2.0f / 3.0f, a, -(1.0f / 6.0f) * b);
+            e1 = __fmaf_rn(1.0f / 6.0f, c, (1.0f / 3.0f) * a);
+            e2 = __fmaf_rn(-(1.0f / 3.0f), g, (5.0f / 6.0f) * c);
+        } else {
+            e0 = __fmaf_rn(-(5.0f / 6.0f), a, (1.0f / 3.0f) * b);
+            e1 = __fmaf_rn(-(1.0f / 3.0f), c, -(1.0f / 6.0f) * a);
+            e2 = __fmaf_rn(1.0f / 6.0f, g, -(2.0f / 3.0f) * c);
+        }
+        const float szero = (z0 ? d0 : 0.0f) + (z1 ? d1 : 0.0f) + (z2 ? d2 : 0.0f);
+        const float den = anyz ? szero : __fmaf_rn(s01, d1, __fmaf_rn(s02, d2, d0));
+        const float inv = __fdividef(1.0f, den);
+        const float w0 = (anyz ? (z0 ? d0 : 0.0f) : d0) * inv;
+        const float w1 = (anyz ? (z1 ? d1 : 0.0f) : d1 * s01) * inv;
+        const float w2 = (anyz ? (z2 ? d2 : 0.0f) : d2 * s02) * inv;
+        const float v = f_c + __fmaf_rn(w0, e0, __fmaf_rn(w1, e1, w2 * e2));
+        if (k == 0) vp = v;
+        else vm = v;
+    }
+}
+
+// FP32 WENO5 face values of model kind KIND, both or one of them.
+template <int KIND>
+__device__ __forceinline__ void weno5_both_mixed(float f_mm, float f_m, float f_c, float f_p, float f_pp, float& vp, float& vm) {
+    if constexpr (KIND == kModelFiveN) weno5_both_f32_nphase(f_mm, f_m, f_c, f_p, f_pp, vp, vm);
+    else weno5_both_f32(f_mm, f_m, f_c, f_p, f_pp, vp, vm);
+}
+template <int KIND>
+__device__ __forceinline__ float weno5_mixed(float f_mm, float f_m, float f_c, float f_p, float f_pp, int side) {
     float vp, vm;
-    weno5_both_f32(f_mm, f_m, f_c, f_p, f_pp, vp, vm);
+    weno5_both_mixed<KIND>(f_mm, f_m, f_c, f_p, f_pp, vp, vm);
     return (side == 1) ? vp : vm;
 }
 

@@ -155,10 +155,9 @@ __device__ __forceinline__ int relax_safeguarded2(double AlphaR[2], const double
 }
 
 // Relax the state U of one cell in place (SixEq<D> layout). FAST (the mixed form): the same FP64
-// root solve with the velocities and phase pressures of the entry state formed by multiplying with
-// reciprocals (one division for 1/rho, the precomputed 1/A_k) and one reciprocal for the volume
-// fraction normalisation, instead of the reference's divisions; the plain form (FAST = false) keeps
-// the reference's operations to the bit.
+// root solve with reciprocals and a square root good to about one unit in the last place (approx_rcp,
+// approx_sqrt) instead of the reference's divisions; the plain form (FAST = false) keeps the reference's
+// operations to the bit.
 template <int D, bool FAST = false>
 __device__ __forceinline__ void relax_pressure(double* U, const Eos& e, double trace, unsigned int* err) {
     using M = SixEq<D>;
@@ -166,7 +165,7 @@ __device__ __forceinline__ void relax_pressure(double* U, const Eos& e, double t
     double W[N];
     if constexpr (FAST) {
         const double rho = U[0] + U[1];
-        const double ir = 1.0 / rho;
+        const double ir = approx_rcp(rho);
         double u[3];
 #pragma unroll
         for (int d = 0; d < D; ++d) u[d] = U[2 + d] * ir;
@@ -229,10 +228,18 @@ __device__ __forceinline__ void relax_pressure(double* U, const Eos& e, double t
         const double aP = ((A1 * A2) + A1 * alpha1) + A2 * alpha2;
         const double bP = (((A1 * B2) * alpha1 + (A2 * B1) * alpha2) - ((A2 + 1.0) * A1) * a1p1) - ((A1 + 1.0) * A2) * a2p2;
         const double cP = ((-B2) * A1) * a1p1 - (B1 * A2) * a2p2;
-        double pR = (-bP + sqrt(bP * bP - (4.0 * aP) * cP)) / (2.0 * aP);
+        const double disc = bP * bP - (4.0 * aP) * cP;
+        double pR;
+        if constexpr (FAST) {
+            pR = (-bP + approx_sqrt(disc)) * approx_rcp(2.0 * aP);
+            alpha1R = fma(pR, alpha1, A1 * a1p1 + B1 * alpha1) * approx_rcp(fma(A1 + 1.0, pR, B1));
+            alpha2R = fma(pR, alpha2, A2 * a2p2 + B2 * alpha2) * approx_rcp(fma(A2 + 1.0, pR, B2));
+        } else {
+            pR = (-bP + sqrt(disc)) / (2.0 * aP);
+            alpha1R = ((A1 * a1p1 + B1 * alpha1) + pR * alpha1) / ((A1 + 1.0) * pR + B1);
+            alpha2R = ((A2 * a2p2 + B2 * alpha2) + pR * alpha2) / ((A2 + 1.0) * pR + B2);
+        }
         pQ = pR;
-        alpha1R = ((A1 * a1p1 + B1 * alpha1) + pR * alpha1) / ((A1 + 1.0) * pR + B1);
-        alpha2R = ((A2 * a2p2 + B2 * alpha2) + pR * alpha2) / ((A2 + 1.0) * pR + B2);
         raw_nan = isnan(alpha1R) || isnan(alpha2R);
         if (isnan(alpha1R) && !isnan(alpha2R))
             alpha1R = 1.0 - alpha2R;
@@ -240,15 +247,17 @@ __device__ __forceinline__ void relax_pressure(double* U, const Eos& e, double t
             alpha2R = 1.0 - alpha1R;
         const double sum = alpha1R + alpha2R;
         if constexpr (FAST) {
-            const double is = 1.0 / sum;
+            const double is = approx_rcp(sum);
             alpha1R *= is;
             alpha2R *= is;
         } else {
             alpha1R /= sum;
             alpha2R /= sum;
         }
-        pR = (((A1 * a1p1 + A2 * a2p2) + B1 * (alpha1 - alpha1R)) + B2 * (alpha2 - alpha2R)) /
-             (A1 * alpha1R + A2 * alpha2R);
+        const double num = ((A1 * a1p1 + A2 * a2p2) + B1 * (alpha1 - alpha1R)) + B2 * (alpha2 - alpha2R);
+        const double den = A1 * alpha1R + A2 * alpha2R;
+        if constexpr (FAST) pR = num * approx_rcp(den);
+        else pR = num / den;
         a1p1R = alpha1R * pR;
         a2p2R = alpha2R * pR;
     }

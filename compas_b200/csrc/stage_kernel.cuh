@@ -850,8 +850,8 @@ __device__ __forceinline__ void stage_tile_faces(const StageArgs& a, int tile, d
                             const float w0 = smem[off[0] + n * str[0]], w1 = smem[off[1] + n * str[1]];
                             const float w2 = smem[off[2] + n * str[2]], w3 = smem[off[3] + n * str[3]];
                             const float w4 = smem[off[4] + n * str[4]], w5 = smem[off[5] + n * str[5]];
-                            wL[n] = weno5_f32(w0, w1, w2, w3, w4, 1);
-                            wR[n] = weno5_f32(w1, w2, w3, w4, w5, -1);
+                            wL[n] = weno5_mixed<M::KIND>(w0, w1, w2, w3, w4, 1);
+                            wR[n] = weno5_mixed<M::KIND>(w1, w2, w3, w4, w5, -1);
                         }
                     }
 #pragma unroll
@@ -1000,13 +1000,6 @@ __host__ __device__ constexpr int segment_cells(int items_per_seg, int cells, in
     return best;
 }
 
-__device__ __forceinline__ void weno5_cell(float f0, float f1, float f2, float f3, float f4, float& vp, float& vm) {
-    weno5_both_f32(f0, f1, f2, f3, f4, vp, vm);
-}
-__device__ __forceinline__ void weno5_cell(double f0, double f1, double f2, double f3, double f4, double& vp, double& vm) {
-    weno5_both(f0, f1, f2, f3, f4, vp, vm);
-}
-
 // Step 2a: the face values of the lines [line0, line0 + LC) along d into the face buffer Fb.
 template <class M, int SCHEME, class T, class PT, int TS, int NT>
 __device__ __forceinline__ void reconstruct_lines(const PT* prim, double* Fb, int d, int line0, int nl_a, int nl_b) {
@@ -1100,7 +1093,8 @@ __device__ __forceinline__ void reconstruct_lines(const PT* prim, double* Fb, in
             if (NSEG * SEG > NCELL && i > TS) break;  // the last segment may be shorter
             const PT f4 = ld(i + 2);
             PT vp, vm;
-            weno5_cell(f0, f1, f2, f3, f4, vp, vm);
+            if constexpr (F32) weno5_both_mixed<M::KIND>(f0, f1, f2, f3, f4, vp, vm);
+            else weno5_both(f0, f1, f2, f3, f4, vp, vm);
             if constexpr (F32) {
                 if (i >= 0) {
                     if (j > 0) reinterpret_cast<float2*>(Fb)[n * FSTR + i * LS + tl] = make_float2(vl, vm);
