@@ -291,3 +291,29 @@ def test_elliptic_solve_converges_on_multiwave_grids(nx, ny):
     lv.close()
     print(f"{nx}x{ny}: solver iterations per step {its}")
     assert max(its) <= 20, its
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 32), (96, 36), (40, 88), (66, 34), (512, 256)])
+def test_implicit_solve_of_the_transposed_flow_is_the_transpose(nx, ny):
+    """The regularisation potential of a flow and of the same flow with x and y exchanged: two solves over
+    different level hierarchies (the single-block coarse cycle's rows, columns and walls change places) that must
+    agree to the solver tolerance; the residual is the solver's, relative to the right-hand side."""
+    torch = _torch()
+    phys, dim, inputs, geom, U = cases.shock_bubble(nx=nx, ny=ny, length=nx / ny, radius=0.15, center=(0.5 * nx / ny, 0.45))
+    inputs = dict(inputs, **{"PhaseField.phase_field": "1", "PhaseField.Mechanism": "CAC-Adv",
+                             "LinearSystem.tol_rel": "1e-12"})
+    V = np.ascontiguousarray(U.transpose(0, 1, 3, 2))
+    V[[2, 3]] = V[[3, 2]]
+    gq = []
+    for W, n, bc in ((U, (nx, ny, 1), (2, 4, 0)), (V, (ny, nx, 1), (4, 2, 0))):
+        p = cb.make_parm(phys, dim, inputs)
+        g = cb.make_geom(n=n, dx=geom["dx"], lo_bc=bc, hi_bc=bc)
+        dev = torch.from_numpy(W.copy()).cuda()
+        cb.FillPatch(p, g, dev)
+        out = [torch.zeros(cb.face_shape(p, g, d, 1), dtype=torch.float64, device="cuda") for d in range(2)]
+        info = cb.PhaseField_GradQPF(p, g, dev, 1e-3, out)
+        assert info[4] < 40 and info[6] <= 1e-12, info
+        gq.append([o.cpu().numpy()[0, 0] for o in out])
+    for d in range(2):
+        a, b = gq[0][d], gq[1][1 - d].T
+        assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(a)  # 1e-12 residual times a condition number of 1e4
