@@ -147,6 +147,8 @@ def test_energy_bound_min_equals_the_reference(dim):
     import torch
 
     p, g, U = _stressed_case(dim, "MUSCL", "air_helium_low_p")
+    if not have_ref(p.physics, p.dim, p.nphase):
+        pytest.skip("reference-header oracle not built")
     # some cells below the bound: lower the energy of a few cells
     V = cb.valid_view(U, p, g)
     V[2 + dim][..., 3] -= 1e-2
