@@ -1392,7 +1392,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                 for (int c = 0; c < NC; ++c) fb[(N + c) * FSTR] = fnc[c];
                 if (fd < TS && gd < nd) cmax_local = dmax(cm, cmax_local);
             }
-            if (a.mode == kModeCmax) continue;  // wave speeds only
+            if (a.mode == kModeCmax) {
+                // wave speeds only: with one halo set resident, the next direction's conversion rewrites the planes
+                // that the limiter of this flux pass reads
+                if constexpr (NHS != D) __syncthreads();
+                continue;
+            }
             __syncthreads();
 
             // 2c. divergence contribution of direction d: (F+ - F-)/dx as the reference divides (FP64 form);

@@ -31,13 +31,14 @@ def _case(model, n, bc, scheme, precision):
     elif model == "six3":
         phys, dim, inputs, geom, U = cases.shock_droplet(n=m)
     else:
-        phys, dim, inputs, geom, U = cases.nphase_bubbles(n=m, nphase=3)
+        phys, dim, inputs, geom, U = cases.nphase_bubbles(n=m, nphase=3, dim=3 if model == "nphase3" else 2)
     gz = 3 if dim == 3 else 0
     nz = n[2] if dim == 3 else 1
     V = U[:, gz:gz + nz, 3:3 + n[1], 3:3 + n[0]].copy()
-    first = 3 if model == "nphase" else 2
+    first = 3 if model.startswith("nphase") else 2
     rho = V[:first].sum(0)
-    amp = {"five2": 0.1, "five3": 20.0, "six2": 20.0, "six3": 20.0, "nphase": 20.0}[model]
+    amp = {"five2": 0.1, "five3": 20.0, "six2": 20.0, "six3": 20.0, "nphase": 20.0,
+           "nphase3": 50.0}[model]
     u = [amp * rng.standard_normal(rho.shape) for _ in range(dim)]
     work = sum(V[first + d] * u[d] + 0.5 * rho * u[d] ** 2 for d in range(dim))
     for d in range(dim):
@@ -152,3 +153,51 @@ def test_weno_quotients_are_the_divisions(kind, scheme):
     cb.compute_dUdt_FV(p, g, dev, dU, cmax=cm)
     assert float(cm.item()) == cmax_ref
     np.testing.assert_array_equal(cb.valid_view(dU.cpu().numpy(), p, g), cb.valid_view(dU_ref, p, g))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [(17, 9, 10), (49, 41, 50)])
+def test_first_wave_speed_of_a_limited_3d_flow(n, precision):
+    """The t = 0 wave-speed pass of the 3D N-phase model, whose flux pass reads the halo planes (the consistent
+    limiter about the cells on either side of a face) and which keeps one direction's planes at a time: a box of
+    few tiles (the large-CTA shape) and one that fills the GPU, as a level, in a batch and as a hierarchy's boxes.
+    The first step's size is that of the largest face speed of compute_dUdt_FV, and in FP64 the C oracle's, every
+    time; a warp that converted the next direction's planes early would change a neighbour's limited state."""
+    import torch
+
+    from compas_b200 import amr
+
+    p, g, U = _case("nphase3", n, "periodic", "WENO5", precision)
+    dev = torch.from_numpy(U.copy()).cuda()
+    cb.FillPatch(p, g, dev)
+    dU, cm = torch.zeros_like(dev), torch.zeros(1, dtype=torch.float64, device="cuda")
+    cb.compute_dUdt_FV(p, g, dev, dU, cmax=cm)
+    cm = float(cm.item())
+    if precision == "fp64":
+        Uf = U.copy()
+        o = Oracle("port", p, g)
+        o.fill_ghosts(Uf)
+        assert cm == o.compute_dudt(Uf)[1]
+    dt = min(p.cfl * g.dx[d] / cm for d in range(3))
+    boxes = amr.hierarchy(n, 3, [], 28)
+    A = cb.Amr(p, g, boxes)
+    batch = cb.Batch(cb.FIVEEQS_NPHASE, 3, id_limiter=5, precision=1 if precision == "mixed" else 0, nphase=3)
+    lv = cb.Level(p, g)
+    lv.set_kernel(0, 0)
+    for _ in range(20):
+        lv.upload(U)
+        lv.advance(1, use_graph=False)
+        lv.sync()
+        assert lv.dts(1)[0] == dt
+        for b, (_, lo, hi) in enumerate(boxes):
+            V = np.zeros((U.shape[0],) + tuple(hi[d] - lo[d] + 7 for d in (2, 1, 0)))
+            V[:, 3:-3, 3:-3, 3:-3] = cb.valid_view(U, p, g)[:, lo[2]:hi[2] + 1, lo[1]:hi[1] + 1, lo[0]:hi[0] + 1]
+            A.upload(b, V)
+        cid = batch.add(p, g, U, max_steps=1)
+        batch.advance(1)
+        assert [i.t for i in batch.poll() if i.id == cid] == [dt]
+        batch.remove(cid)
+    A.advance(1)
+    assert A.dts(1)[0] == dt
+    for h in (A, batch, lv):
+        h.close()
