@@ -499,11 +499,19 @@ __device__ __forceinline__ void stage_epilogue(const StageArgs& a, const double 
 // CTA max of the face wave speeds -> one atomic.
 template <int NT>
 __device__ __forceinline__ void cta_cmax(unsigned long long* cmax, double v) {
+    constexpr int TAIL = NT % 32;  // lanes of a partial last warp (144, 272 and 136 threads)
     const int tid = threadIdx.x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __shared__ double wmax[32];
     const int w = tid >> 5, lane = tid & 31;
+    if (TAIL == 0 || w < NT / 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    } else {
+        // a lane whose partner does not exist keeps its own value; lane 0 still sees every live lane
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            v = dmax(v, __shfl_sync((1u << TAIL) - 1u, v, (lane ^ o) < TAIL ? lane ^ o : lane));
+    }
+    __shared__ double wmax[32];
     if (lane == 0) wmax[w] = v;
     __syncthreads();
     if (tid == 0) {

@@ -201,3 +201,29 @@ def test_first_wave_speed_of_a_limited_3d_flow(n, precision):
     assert A.dts(1)[0] == dt
     for h in (A, batch, lv):
         h.close()
+
+
+@pytest.mark.parametrize("scheme", ["WENO5", "MUSCL"])
+def test_wave_speed_of_every_part_of_a_tile_counts(scheme):
+    """One fast cell at places over a 16^2 tile, whose faces fall to different warps of the CTA, the partial last
+    one of the 144-, 272- and 136-thread shapes among them: the second step's size, which the largest face speed
+    of the first step's stages sets, is the same for every launch shape, and with WENO5 in FP64 the C oracle's."""
+    rng = np.random.default_rng(5)
+    phys, dim, inputs, geom, _ = cases.shock_bubble(nx=16, ny=16, length=1.0)
+    for i, j in [(0, 0), (7, 0), (8, 5), (7, 8), (8, 15), (15, 15), (3, 8), (15, 2)]:
+        V = np.empty((6, 1, 16, 16))
+        rho, u = 1.0 + 0.1 * rng.random((1, 16, 16)), 0.1 * rng.standard_normal((2, 1, 16, 16))
+        u[:, 0, j, i] += 2.0
+        V[0], V[1], V[5] = 0.75 * rho, 0.25 * rho, 0.5
+        V[2:4] = rho * u
+        V[4] = 2.5 + 0.5 * rho * (u * u).sum(0)
+        for precision in ("fp64", "mixed"):
+            p = cb.make_parm(phys, dim, dict(inputs, **{"FiniteVolume.Scheme": scheme, "compas_b200.precision": precision}))
+            g = cb.make_geom(n=(16, 16, 1), dx=geom["dx"], lo_bc=(2, 2, 0), hi_bc=(2, 2, 0))
+            U = np.zeros(cb.padded_shape(p, g))
+            cb.valid_view(U, p, g)[...] = V
+            dts = [_advance(p, g, U, 2, shape)[1] for shape in range(3)]
+            np.testing.assert_array_equal(dts[1], dts[0])
+            np.testing.assert_array_equal(dts[2], dts[0])
+            if precision == "fp64" and scheme == "WENO5":  # the C oracle has no MUSCL
+                np.testing.assert_array_equal(dts[0], Oracle("port", p, g).advance(U.copy(), 2)[1])
