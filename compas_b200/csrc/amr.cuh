@@ -338,6 +338,10 @@ __device__ void amr_face_flux(const double* U, const Grid& g, int d, int i, int 
             M::prim2cons(UR, WfR, e, err);
             riemann<M>(id_riemann, F, fnc, cm, UL, UR, e, d, id_k, err);
         } else {
+            if (e.C1 > 0.0 || e.C2 > 0.0) {
+                covolume_check<M>(wL, e, err);
+                covolume_check<M>(wR, e, err);
+            }
             float cmf;
             mixed_riemann<M>(id_riemann, F, fnc, cmf, wL, wR, e, d, id_k, MixedState<M>{wL, wR, e});
         }

@@ -247,3 +247,29 @@ def test_rejects_thinc_and_bad_mode():
     pt = cb.make_parm(cb.FIVEEQS, 2, {"FiniteVolume.THINC": "1"})
     with pytest.raises(cb.CompasError):
         cb.face_fluxes(pt, g, Ud, F)
+
+
+@pytest.mark.parametrize("scheme", ["WENO5", "WENO5B", "MUSCL-MC"])
+@pytest.mark.parametrize("physics", [cb.FIVEEQS, cb.SIXEQS], ids=["fiveeq", "sixeq"])
+def test_covolume_violation_is_reported_in_both_forms(physics, scheme):
+    """NASG face states of a phase with 1 - b rho <= 0 set the status bit, as the right-hand side's do; phases
+    within their covolume set none."""
+    import torch
+
+    _, dim, inputs, geom, U = cases.advected_interface(n=16, dim=2, physics=physics)
+    V = cb.valid_view(U, cb.make_parm(physics, dim, inputs), cb.make_geom(**geom))
+    rho2 = float((V[1] / (1.0 - V[-1])).max())
+    for factor, status in ((0.5, 0), (2.0, cb.ERR_COVOLUME)):
+        for precision in ("fp64", "mixed"):
+            p = cb.make_parm(physics, dim, dict(inputs, **{
+                "FiniteVolume.Scheme": scheme, "compas_b200.precision": precision, "prob.EOS.EOS": 3,
+                "prob.EOS.b_2": factor / rho2}))
+            g = cb.make_geom(**geom)
+            Ud = _dev(torch, U)
+            cb.FillPatch(p, g, Ud)
+            F = [torch.zeros(cb.face_shape(p, g, d, cb.parm_nstate(p)), dtype=torch.float64, device="cuda") for d in range(2)]
+            err = torch.zeros(2, dtype=torch.int32, device="cuda")
+            cb.face_fluxes(p, g, Ud, F, err=err)
+            cb.compute_dUdt_FV(p, g, Ud, torch.zeros_like(Ud), err=err[1:])
+            got = err.cpu().tolist()
+            assert [e & cb.ERR_COVOLUME for e in got] == [status, status], (precision, factor, got)
