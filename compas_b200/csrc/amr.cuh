@@ -337,6 +337,19 @@ __device__ void amr_face_flux(const double* U, const Grid& g, int d, int i, int 
             M::prim2cons(UL, WfL, e, err);
             M::prim2cons(UR, WfR, e, err);
             riemann<M>(id_riemann, F, fnc, cm, UL, UR, e, d, id_k, err);
+        } else if constexpr (SCHEME == 2) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                WfL[n] = wL[n];
+                WfR[n] = wR[n];
+            }
+            M::prim2cons(UL, WfL, e, err);
+            M::prim2cons(UR, WfR, e, err);
+            float cmf;
+            mixed_riemann<M>(id_riemann, F, fnc, cmf, wL, wR, e, d, id_k, [&](bool left, double* Uf) {
+#pragma unroll
+                for (int n = 0; n < N; ++n) Uf[n] = left ? UL[n] : UR[n];
+            });
         } else {
             if (e.C1 > 0.0 || e.C2 > 0.0) {
                 covolume_check<M>(wL, e, err);

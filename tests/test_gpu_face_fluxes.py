@@ -273,3 +273,38 @@ def test_covolume_violation_is_reported_in_both_forms(physics, scheme):
             cb.compute_dUdt_FV(p, g, Ud, torch.zeros_like(Ud), err=err[1:])
             got = err.cpu().tolist()
             assert [e & cb.ERR_COVOLUME for e in got] == [status, status], (precision, factor, got)
+
+
+@pytest.mark.parametrize("riemann", ["HLLC", "HLL"])
+@pytest.mark.parametrize("scheme", ["MUSCL-MC", "WENO3", "WENO3B", "WENO5", "WENO5B"])
+@pytest.mark.parametrize("physics", [cb.FIVEEQS, cb.SIXEQS], ids=["fiveeq", "sixeq"])
+def test_mixed_face_fluxes_are_the_stage_kernels_bits(physics, scheme, riemann):
+    """The mixed form's fluxes for the registers and those of the stage kernel, to the bit. The flow is uniform along
+    y, whose flux differences are then exactly 0, so the right-hand side of a mass, a momentum or the five-equation
+    energy is the one product -(F_hi - F_lo) (1 / dx) (the kernel's sum over directions is a fused multiply-add otherwise)."""
+    import torch
+
+    _, dim, inputs, geom, U = cases.advected_interface(n=24, dim=2, physics=physics)
+    U = np.ascontiguousarray(np.broadcast_to(U[:, :, 15:16, :], U.shape))
+    p = cb.make_parm(physics, dim, dict(inputs, **{"FiniteVolume.Scheme": scheme, "Physics.RiemannSolver": riemann,
+                                                    "compas_b200.precision": "mixed"}))
+    g = cb.make_geom(**geom)
+    rng = np.random.default_rng(3)
+    V = cb.valid_view(U, p, g)
+    u = 700.0 * rng.standard_normal((2, 1, 1, V.shape[-1]))  # kinetic energies of the size of the internal ones
+    work = (V[2:4] * u).sum(0) + 0.5 * (V[0] + V[1]) * (u * u).sum(0)
+    V[2:4] += (V[0] + V[1]) * u
+    if physics == cb.SIXEQS:
+        V[4] += V[0] / (V[0] + V[1]) * work
+        V[5] += V[1] / (V[0] + V[1]) * work
+    else:
+        V[4] += work
+    Ud = _dev(torch, U)
+    cb.FillPatch(p, g, Ud)
+    dU = torch.zeros_like(Ud)
+    cb.compute_dUdt_FV(p, g, Ud, dU)
+    F, _ = _faces(torch, p, g, area=False, U=Ud)
+    got = cb.valid_view(dU.cpu().numpy(), p, g)
+    assert np.all(np.isfinite(got))
+    for c in range(4 if physics == cb.SIXEQS else 5):
+        np.testing.assert_array_equal(-((F[0][c, ..., 1:] - F[0][c, ..., :-1]) * (1.0 / g.dx[0])), got[c])
