@@ -568,18 +568,26 @@ __device__ __forceinline__ double face_speed(const double* UL, const double* UR,
     return dmax(q[0], q[1]);
 }
 
-// The same of a two-phase model in the mixed form.
+// The same of a two-phase model in the mixed form (the LLF and HLL solvers square and sum without fused steps).
 template <class M>
-__device__ __forceinline__ float face_speed_mixed(const float* wL, const float* wR, const Eos& e, int id_k) {
+__device__ __forceinline__ float face_speed_mixed(int id_riemann, const float* wL, const float* wR, const Eos& e, int id_k) {
     float q[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const float* w = s ? wR : wL;
-        float c, k = __fmaf_rn(w[2], w[2], w[3] * w[3]);
-        if (M::D == 3) k = __fmaf_rn(w[4], w[4], k);
+        float c, u;
         if constexpr (M::KIND == kModelSix) c = sixeq_c_f32<M::D>(w, e);
         else c = fiveeq_c_f32<M::D>(w, e, id_k);
-        q[s] = c + sqrt_ftz(k);
+        if (id_riemann == 2) {
+            float k = __fmaf_rn(w[2], w[2], w[3] * w[3]);
+            if (M::D == 3) k = __fmaf_rn(w[4], w[4], k);
+            u = sqrt_ftz(k);
+        } else {
+            float k = w[2] * w[2] + w[3] * w[3];
+            if (M::D == 3) k += w[4] * w[4];
+            u = sqrtf(k);
+        }
+        q[s] = c + u;
     }
     return fmaxf(q[0], q[1]);
 }
@@ -1386,7 +1394,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                         }
                         float cmf;
                         if (a.mode == kModeCmax) {
-                            cm = face_speed_mixed<M>(wL, wR, a.e, a.id_k);
+                            cm = face_speed_mixed<M>(a.riemann, wL, wR, a.e, a.id_k);
                             if (fd < TS && gd < nd) cmax_local = dmax(cm, cmax_local);
                             continue;
                         }

@@ -227,3 +227,41 @@ def test_wave_speed_of_every_part_of_a_tile_counts(scheme):
             np.testing.assert_array_equal(dts[2], dts[0])
             if precision == "fp64" and scheme == "WENO5":  # the C oracle has no MUSCL
                 np.testing.assert_array_equal(dts[0], Oracle("port", p, g).advance(U.copy(), 2)[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("riemann", ["LLF", "HLL", "HLLC"])
+@pytest.mark.parametrize("model", ["five2", "six2", "five3", "six3", "nphase"])
+def test_first_step_size_is_the_right_hand_sides_wave_speed(model, riemann, precision):
+    """The t = 0 pass forms the face speeds without the fluxes: bit for bit those of the Riemann solver in use, for
+    supersonic drifts (where a unit in the last place of |u| shows in c + |u|, in one of some dozen drifts)."""
+    import torch
+
+    rng = np.random.default_rng(11)
+    n = (12, 9, 1) if model in ("five2", "six2", "nphase") else (9, 8, 5)
+    p, g, U0 = _case(model, n, "periodic", "WENO5", precision)
+    p.id_riemann = {"LLF": 0, "HLL": 1, "HLLC": 2}[riemann]
+    lv = cb.Level(p, g)
+    lv.set_kernel(0, 0)
+    for _ in range(60):
+        U = U0.copy()
+        V = cb.valid_view(U, p, g)
+        first = 3 if model == "nphase" else 2
+        rho = V[:first].sum(0)
+        drift = (6.0 if model == "five2" else 6000.0) * (1.0 + 0.3 * rng.random(3))
+        work = sum(drift[d] * (V[first + d] + 0.5 * rho * drift[d]) for d in range(p.dim))
+        for d in range(p.dim):
+            V[first + d] += rho * drift[d]
+        if p.physics == cb.SIXEQS:
+            V[first + p.dim] += V[0] / rho * work
+            V[first + p.dim + 1] += V[1] / rho * work
+        else:
+            V[first + p.dim] += work
+        dev = torch.from_numpy(U).cuda()
+        cb.FillPatch(p, g, dev)
+        cm = torch.zeros(1, dtype=torch.float64, device="cuda")
+        cb.compute_dUdt_FV(p, g, dev, torch.zeros_like(dev), cmax=cm)
+        lv.upload(U)
+        lv.advance(1, use_graph=False)
+        assert lv.dts(1)[0] == min(p.cfl * g.dx[d] / float(cm.item()) for d in range(p.dim))
+    lv.close()
