@@ -798,18 +798,27 @@ __device__ __forceinline__ void weno5_cand(double f_mm, double f_m, double f_c, 
 
 // FP64 quotients without the range handling of a division, for operands that the caller knows to be
 // positive and far from over- and underflow.
-// approx_rcp: within about one unit in the last place of 1/b, the hardware's 20-bit estimate refined by the
-// cubic step y (1 + e + e^2), e = 1 - b y. refine_rcp: the correctly rounded 1/b from a y within a few units
+// near_rcp: within one unit in the last place of 1/b, the hardware's 20-bit estimate refined by the cubic
+// step y (1 + e + e^2), e = 1 - b y. refine_rcp: the correctly rounded 1/b from a y within a few units
 // of it: a first step rounded upwards, so that the result is within one unit and not below where b's
 // significand is all ones, then P. Markstein's step y + y (1 - b y), whose residual is exact in an FMA
 // ("Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).
 // div_rn: the correctly rounded a/b from y = 1/b so rounded, by the same paper's q + (a - b q) y. One
 // reciprocal serves every quotient over the same denominator, and none of it branches.
-__device__ __forceinline__ double approx_rcp(double b) {
+__device__ __forceinline__ double near_rcp(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     const double e = fma(-b, y, 1.0);
     return fma(fma(e, e, e), y, y);
+}
+// near_rcp for any b (mixed form): 0 gives infinity and infinity 0 with their signs, as 1/b does (the step's
+// residual is NaN there and the estimate stands); a subnormal b reads as 0.
+__device__ __forceinline__ double approx_rcp(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    const double r = fma(fma(e, e, e), y, y);
+    return (r == r) ? r : y;
 }
 __device__ __forceinline__ double refine_rcp(double b, double y) {
     y = __fma_ru(fma(-b, y, 1.0), y, y);
@@ -827,15 +836,16 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-// sqrt(x) within about one unit in the last place (mixed form; NaN for x < 0): two Newton steps
-// y (3 - x y^2)/2 on the hardware's estimate of 1/sqrt(x), then x y with its residual folded in.
+// sqrt(x) within one unit in the last place (mixed form; NaN for x < 0): one Newton step y (3 - x y^2)/2 on the
+// hardware's estimate of 1/sqrt(x), which leaves some 2^-40, then x y with its residual x - s^2 folded in, which
+// squares that. The residual of 0 and of infinity is NaN and they give themselves, as does a positive subnormal x.
 __device__ __forceinline__ double approx_sqrt(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     y = y * fma(-0.5 * x, y * y, 1.5);
     const double s = x * y;
     const double r = fma(fma(-s, s, x), 0.5 * y, s);
-    return (x > 0.0) ? r : ((x < 0.0) ? __longlong_as_double(0x7ff8000000000000ll) : x);
+    return (x < 0.0) ? __longlong_as_double(0x7ff8000000000000ll) : ((r == r) ? r : x);
 }
 
 // Weights of the right face (wp) and the left face (wm) of the centre cell. Where the indicators lie within
@@ -863,7 +873,7 @@ __device__ __forceinline__ void weno5_weights(double f_mm, double f_m, double f_
                    h2 = (unsigned)__double2hiint(IS2);
     constexpr unsigned LO = (1023u - 240u) << 20, HI = (1023u + 240u) << 20;
     if (min(min(h0, h1), h2) >= LO && max(max(h0, h1), h2) < HI) {
-        const double y0 = approx_rcp(IS0), y1 = rcp_rn(IS1), y2 = rcp_rn(IS2);
+        const double y0 = near_rcp(IS0), y1 = rcp_rn(IS1), y2 = rcp_rn(IS2);
         const double IS01 = div_rn(IS0, IS1, y1), IS02 = div_rn(IS0, IS2, y2), IS12 = div_rn(IS1, IS2, y2);
         // 1/IS01 from its close approximation IS1/IS0, and so on
         const double IS10 = refine_rcp(IS01, IS1 * y0), IS20 = refine_rcp(IS02, IS2 * y0), IS21 = refine_rcp(IS12, IS2 * y1);
