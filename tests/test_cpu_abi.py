@@ -6,6 +6,7 @@ import re
 import pytest
 
 import compas_b200 as cb
+from compas_b200 import cases
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -108,6 +109,15 @@ def test_nc_terms_and_face_shapes():
     assert cb.face_shape(p, g, 0, 8) == (8, 7, 6, 6)
     assert cb.face_shape(p, g, 1, 3) == (3, 7, 7, 5)
     assert cb.face_shape(p, g, 2, 8) == (8, 8, 6, 5)
+
+
+def test_amr_refuses_bad_boxes_before_it_needs_a_device():
+    phys, dim, inputs, geom, _ = cases.shock_bubble(nx=32, ny=16)
+    p, g = cb.make_parm(phys, dim, inputs), cb.make_geom(**geom)
+    for box, why in [((0, (0, 0, 0), (40, 15, 0)), "outside its level"), ((0, (0, 0, 0), (1, 15, 0)), "at least ng cells")]:
+        with pytest.raises(cb.CompasError, match=why) as e:
+            cb.Amr(p, g, [box])
+        assert e.value.code == -1  # COMPAS_B200_EARG
 
 
 def test_amr_interpolater_key():
