@@ -116,6 +116,22 @@ def test_every_shape_gives_the_oracles_bits(model, n, bc, scheme):
     assert np.linalg.norm(mix[-1] - ref[-1]) <= 1e-5 * np.sqrt(ref[-1].size)
 
 
+@pytest.mark.parametrize("scheme", ["WENO5", "WENO5B"])
+@pytest.mark.parametrize("model,n,bc", [("five2", n, "mixed") for n in SIZES2] + [("nphase", n, "walls") for n in SIZES2] +
+                         [("six2", n, "walls") for n in SIZES2] + [("five3", n, "mixed") for n in SIZES3] +
+                         [("nphase3", n, "walls") for n in SIZES3] + [("six3", n, "outflow") for n in SIZES3])
+def test_every_shape_gives_the_same_mixed_bits(model, n, bc, scheme):
+    """The mixed form's launch shapes split lines into other segments and carry face values across their ends, but
+    every face takes the same operations: the same bits, at the ragged and odd sizes."""
+    p, g, U = _case(model, n, bc, scheme, "mixed")
+    ref, dts_ref = _advance(p, g, U, 2, 0)
+    assert np.all(np.isfinite(ref))
+    for shape in (1, 2):
+        got, dts = _advance(p, g, U, 2, shape, order=shape % 2)
+        np.testing.assert_array_equal(dts, dts_ref)
+        np.testing.assert_array_equal(got, ref, err_msg=f"shape {shape}")
+
+
 @pytest.mark.parametrize("kind", ["ulps", "ulps_jump", "zero_runs", "wide"])
 @pytest.mark.parametrize("scheme", ["WENO5", "WENO5B"])
 def test_weno_quotients_are_the_divisions(kind, scheme):
