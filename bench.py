@@ -152,9 +152,9 @@ def measured_peaks():
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the mixed stage kernel, from
 # one ncu capture of the 128^3 shock-droplet (three launches, one per RK stage, averaged) scaled by the
 # 8x cells of a 256^3 launch; a measured constant, not recomputed by this run.
-STAGE_TRAFFIC_BYTES = 2.99e9
-STAGE_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, mixed stage kernel (TMA form, NT 288), "
-                        "128^3 shock-droplet, mean of the three RK stages (373.7 MB), x8 for 256^3")
+STAGE_TRAFFIC_BYTES = 2.85e9
+STAGE_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, mixed stage kernel (320 threads, 2 CTAs per SM, "
+                        "no TMA), 128^3 shock-droplet, mean of the three RK stages (356.1 MB), x8 for 256^3")
 
 
 def _reference_oracle(n):
@@ -199,9 +199,10 @@ STAGE_FLOPS_SOURCE = ("static count of the formulas per cell and RK stage, SIXEQ
                       "+ - * / sqrt = 1 operation")
 # Executed floating-point operations per cell and RK stage, from ncu's SASS operation counters
 # (smsp__sass_thread_inst_executed_op_{f,d}{add,mul,fma}_pred_on.sum, FMA = 2) of the 128^3 capture of
-# each form's stage kernel, mean of the three RK stages. They exceed the static counts by the
-# instruction sequences of the divisions and square roots (reciprocal refinement, range checks).
-STAGE_FLOPS_EXECUTED = {"mixed": {"fp32": 3502, "fp64": 1104}, "fp64": {"fp32": 955, "fp64": 17342}}
+# each form's stage kernel, mean of the three RK stages. The mixed form's FP32 count lies below the static
+# one, which forms every face value's weights alone; the FP64 form's exceeds it by the steps of its correctly
+# rounded quotients and square roots.
+STAGE_FLOPS_EXECUTED = {"mixed": {"fp32": 2009, "fp64": 844}, "fp64": {"fp32": 275, "fp64": 11866}}
 STAGE_FLOPS_EXECUTED_SOURCE = ("ncu SASS operation counters (add, mul, fma x2) of the 128^3 stage-kernel capture, "
                                "mean of the three RK stages")
 
