@@ -188,7 +188,7 @@ def cpu_baseline(n, steps):
 
 # Algorithmic floating-point operations per cell and RK stage of the 256^3 shock-droplet (SIXEQS 3D,
 # WENO5 + HLLC + relaxation), a static count of the formulas with each +, -, *, / and sqrt counted as
-# one operation (the per-function table is in DESIGN.md): per face 16 WENO5 calls (79 each), two
+# one operation: per face 16 WENO5 calls (79 each), two
 # primitive-to-conservative conversions (30), the HLLC flux with its conversions, fluxes and sound
 # speeds (437); per cell three faces, one cell conversion (30), the divergence (88), the
 # non-conservative terms (14), the stage combination (32 on average) and the closed-form relaxation

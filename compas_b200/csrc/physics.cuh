@@ -345,7 +345,9 @@ struct FiveEq {
         const double S_Star = (((pR - pL) + (rhoL * VL) * (SL - VL)) - (rhoR * VR) * (SR - VR)) /
                               (rhoL * (SL - VL) - rhoR * (SR - VR));
         // The reference blends both sides' star states with the weights (1 + sign S*)/2 and (1 - sign S*)/2; a
-        // side of weight 0 adds nothing, so only the upwind one is formed, and both where S* is 0 (or NaN).
+        // side of weight 0 adds nothing, so only the upwind one is formed, and both where S* is 0 (or NaN). The
+        // value is the blend's to the bit except where the other side's star state is infinite or NaN (vacuum),
+        // which the blend's 0 times infinity makes NaN and which is ignored here.
         const bool left = S_Star > 0.0, both = !(left || S_Star < 0.0);
         auto side = [&](bool lt, double* F, double& vel, double& dvel) {
             const double V = lt ? VL : VR, p = lt ? pL : pR, rho = lt ? rhoL : rhoR, SK = lt ? SL : SR;
@@ -780,8 +782,9 @@ __device__ __forceinline__ void sixeq_hllc_mixed(double* Fout, double* fnc, floa
 // ------------------------------------------------------------------------------------------------
 // WENO5 face values (WENO5.H:12-75), epsilon-free weights from smoothness ratios with a NaN guard.
 // side = +1: value at the right face of the centre cell c; side = -1: at its left face. The two faces
-// of a cell share the indicators, the ratios and their squares, which are formed once for both (12
-// divisions for two face values; a face value formed alone takes 9), with the reference's operations.
+// of a cell share the indicators, the ratios and their squares, which are formed once for both: 12 quotients
+// (6 ratios, 6 weights) for two face values where a face value formed alone takes 9, each the correctly rounded
+// value of the reference's division (weno5_weights; divisions themselves on its fallback path only).
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void weno5_cand(double f_mm, double f_m, double f_c, double f_p, double f_pp, int side,
                                            double q[3]) {
@@ -1056,9 +1059,9 @@ __device__ __forceinline__ void weno5b_masses(const double* ar1, const double* a
 //
 // Indicators: three times the reference's (integer coefficients; only ratios enter), each a positive
 // definite form of two differences (smallest eigenvalue 0.73), so rounding cannot make one negative.
-// kWenoFloor, far below the square of any FP32 difference of a resolved field, stands in for zero: all
-// indicators zero gives the linear weights, some zero gives those stencils their share of them, as the
-// reference's NaN guard does. Ratios are clamped at 1e18, where the weights are 0 or 1 to FP32
+// kWenoFloor stands in for zero: all indicators zero gives the linear weights, some zero gives those stencils
+// their share of them, as the reference's NaN guard does. It gives the weights a scale: differences below some
+// 1e-18 count as none (fields of order 1e-11 and more resolve no such difference in FP32). Ratios are clamped at 1e18, where the weights are 0 or 1 to FP32
 // precision, so that the squares stay finite.
 // ------------------------------------------------------------------------------------------------
 constexpr float kWenoFloor = 1.0e-36f;
@@ -1111,7 +1114,8 @@ __device__ __forceinline__ void weno5_both_f32(float f_mm, float f_m, float f_c,
     vm = f_c + weno5_corr_f32(g, c, a, b, -1, wm);
 }
 
-// The N-phase model's FP32 weights: the same ratio form with the reference's coefficients as they stand and
+// The FP32 weights of the five-equation N-phase model with plain WENO5 (its WENO5B, and the six-equation N-phase
+// model, take those above): the same ratio form with the reference's coefficients as they stand and
 // the vanishing indicators told apart by comparisons. Its flows (sharp interfaces under a limiter that
 // switches on slope sums of 1e-10) carry a change of rounding in these weights to 5e-6 of the state within 20
 // small-grid steps, so they keep the rounding they have had; the two faces share indicators and ratios.
@@ -1264,7 +1268,7 @@ __device__ __forceinline__ float muscl_face_f32(float f_m, float f_c, float f_p,
     return __fmaf_rn((float)side * 0.5f, s, f_c);
 }
 
-// WENO3 in FP32 in the correction form of weno5_f32 (f_c plus the weighted corrections), the weights
+// WENO3 in FP32 in the correction form of weno5_corr_f32 (f_c plus the weighted corrections), the weights
 // from the ratio of the indicators with one reciprocal.
 // Weight of the left candidate from the undivided differences a = f_c - f_m, b = f_p - f_c.
 __device__ __forceinline__ float weno3_w0_f32(float a, float b, int side) {

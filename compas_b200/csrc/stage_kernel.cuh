@@ -1101,7 +1101,7 @@ __device__ __forceinline__ void reconstruct_lines(const PT* prim, double* Fb, in
         PT f0 = ld(i0 - 2), f1 = ld(i0 - 1), f2 = ld(i0), f3 = ld(i0 + 1);
         PT vl = 0;  // left value of the current cell's low face, from the cell before
         // FP32: unrolled, so that squares and products of differences carry over from cell to cell. FP64: a
-        // cell is some 400 instructions (12 divisions); rolled, the loop stays in the instruction cache.
+        // cell is some 400 instructions (12 quotients); rolled, the loop stays in the instruction cache.
         constexpr int UNROLL = F32 ? SEG : 1;
 #pragma unroll UNROLL
         for (int j = 0; j < SEG; ++j) {
@@ -1143,7 +1143,8 @@ __device__ __forceinline__ void reconstruct_lines(const PT* prim, double* Fb, in
 // The work of one CTA on tile `tile` of the box described by `a` (tiles numbered x fastest).
 //
 // What bounds it: instruction issue, not memory (DRAM traffic is the algorithmic bytes). Forming both face
-// values of a cell at once halves the smoothness indicators and, in FP64, takes 12 divisions instead of 18.
+// values of a cell at once halves the smoothness indicators and, in FP64, takes 12 quotients
+// instead of 18.
 template <class M, int SCHEME, bool MIX, int VAR, int TX, int TY, int TZ, int NT, int CTAS>
 __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double* smem_d, const TmaMaps* tm = nullptr) {
     static_assert(TX == TY && (M::D == 2 ? TZ == 1 : TZ == TX), "tiles are cubes (squares in 2D)");

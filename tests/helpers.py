@@ -10,7 +10,7 @@ def oracle_kind(physics, dim, nphase=2):
 
 
 def rel_linf(a, b):
-    """max |a - b| / max |b| per component (the parity norm of the north star)."""
+    """max |a - b| / max |b| per component (the parity norm)."""
     out = []
     for c in range(a.shape[0]):
         den = float(np.max(np.abs(b[c])))

@@ -5,7 +5,7 @@ Both sides run the same fixed hierarchy (refinement ratio 2, subcycling, flux re
 five-equation non-conservative alpha1 source or the six-equation phase-energy and alpha1 terms and the
 relaxation of the refluxed cells, average-down), the same coarse-fine interpolation and
 the reference's own face arithmetic, so the plain FP64 form is compared to the bit (the asserted bound
-is the north star's 1e-11 relative L-infinity per field and box). The coarse-fine operations follow
+is 1e-11 relative L-infinity per field and box). The coarse-fine operations follow
 AMReX's documented semantics on both sides; AMReX itself is not in the image, so they are not pinned
 by the reference. Also: one level of several boxes equals the single-box level; the composite-grid
 totals of mass, momentum and energy are conserved to round-off on a periodic domain; every level's

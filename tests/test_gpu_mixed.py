@@ -1,7 +1,7 @@
 """The mixed-precision form (FP32 reconstruction; FP64 pressure recovery, Riemann solver, stage
 accumulation and relaxation) against the FP64 path, which is the reference's arithmetic to the bit.
 
-The bound is the north star's: relative L1 error (sum |a - b| / sum |b|) in the densities and the
+The bound: relative L1 error (sum |a - b| / sum |b|) in the densities and the
 volume fraction <= 1e-5 against the FP64 result after the stated steps; every field's error is
 printed. Mass, momentum and energy stay conserved to round-off because each face flux is computed
 once and used by both neighbouring cells, whatever its precision."""

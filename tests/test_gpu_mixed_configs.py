@@ -3,7 +3,7 @@ counts, and the plain FP64 form with the Phase-Field step against the reference-
 few hundred steps.
 
   * 3D shock-droplet (the six-equation configuration), 200 steps: relative L1 of the partial densities
-    and of the volume fraction <= 1e-5 (the north star's bound); 128^3, the 256^3 configuration halved
+    and of the volume fraction <= 1e-5 (the stated bound); 128^3, the 256^3 configuration halved
     (the 256^3 figure after 200 steps is printed by bench.py);
   * 2D shock-helium-bubble with the CAC-Adv Phase-Field step (the five-equation configuration:
     2048 x 1024, WENO5B + HLLC, eta = dx), 1000 steps, both forms: relative L1 of the partial densities

@@ -3,7 +3,7 @@
 The plain FP64 form reproduces the reference's arithmetic - WENO5 in primitive variables, the
 consistent limiter of the partial densities and volume fractions, HLLC, the Kapila terms of every
 volume fraction - so the right-hand side, the face wave speed and whole level advances are compared
-to the bit against the reference-header oracle (the asserted bound is the north star's 1e-11
+to the bit against the reference-header oracle (the asserted bound is 1e-11
 relative L-infinity per field). Cases: the triple point of the serving workload (NPHASE = 3, sharp
 interfaces, reflecting walls), advected bubbles with 2, 3 and 4 phases, the Kapila K term and the
 NASG covolume, a 3D case; the box-list (batched) form against the single-box form; and the mixed

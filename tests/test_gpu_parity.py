@@ -1,7 +1,7 @@
 """Parity of the CUDA path (through the C ABI) with the CPU oracle on identical initial data.
 
 The plain FP64 form evaluates the reference's formulas in the reference's order with FMA
-contraction off, so the expected difference is zero; the asserted bound is the north star's
+contraction off, so the expected difference is zero; the asserted bound is
 1e-11 relative L-infinity per field, and every test also reports the measured difference.
 """
 import numpy as np

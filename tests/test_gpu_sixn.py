@@ -8,7 +8,7 @@ bounded partial densities and volume fractions), the model's HLLC / HLL / LLF fl
 non-conservative terms alpha_k div u and alpha_k p_k div u, and the Newton pressure relaxation with its
 safeguarded fallback after every stage. The right-hand side, the face wave speed and whole level
 advances are compared to the bit against the reference-header oracle (oracle/_ref/libref_6eqn*); the
-asserted bound is the north star's 1e-11 relative L-infinity per field. Cases: a Mach 1.1 water shock
+asserted bound is 1e-11 relative L-infinity per field. Cases: a Mach 1.1 water shock
 on an air bubble (and a helium bubble with three phases), after the reference's
 ShockBubble-WaterAir-6Eq-Nphase example, in pressure equilibrium and out of it, with the NASG
 covolume, with a trace threshold that sends phases through the safeguarded relaxation, and in 3D.

@@ -2,7 +2,7 @@
 
 The reference's THINC face value uses exp, log and tanh; the CUDA path calls CUDA's double-precision
 exp, log and tanh, which may differ from the host C library in the last bit. Where a case does not
-amplify such a difference the bound is the north star's 1e-11 relative L-infinity per field. The
+amplify such a difference the bound is 1e-11 relative L-infinity per field. The
 THINC switch is discontinuous (a face changes scheme when a strict comparison of volume fractions
 flips) and the six-equation relaxation is a root solve, so some cases amplify a last-bit difference
 far above 1e-11. For every case the test therefore measures that amplification on the oracle itself
