@@ -1155,6 +1155,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
     static_assert(!PFX || M::KIND == kModelFive || M::KIND == kModelSix, "the Phase-Field kernel is the two-phase models'");
     constexpr bool NPH = (M::KIND == kModelFiveN);
     constexpr bool SXN = (M::KIND == kModelSixN);
+    // N-phase WENO5: the consistent limiter about the stencil centres f-1 and f, whose primitives the flux pass
+    // then reads (WENO5B bounds its face values instead)
+    constexpr bool LIMIT = NPH && SCHEME == 5;
     using PT = typename std::conditional<MIX, float, double>::type;
     constexpr int TS = TX;
     using T = ReconShape<M, TS, PT, TMA, PFX, CTAS>;
@@ -1334,9 +1337,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                         for (int n = 0; n < N; ++n) W[n] = fb[(N + n) * FSTR];
                         M::prim2cons(UR, W, a.e, err);
                     }
-                    if constexpr (NPH && SCHEME == 5) {
-                        // N-phase WENO5: the consistent limiter about the stencil centres f-1 and f (WENO5B
-                        // bounds its face values instead)
+                    if constexpr (LIMIT) {
                         const int b = T::base(d, t), h = T::halo(d, t), sd = T::stride(d);
                         M::consistent_limit(UL, prim + T::cell(b, sd, h, fd - 1), CSTR, dxd, 1, a.e, err);
                         M::consistent_limit(UR, prim + T::cell(b, sd, h, fd), CSTR, dxd, -1, a.e, err);
@@ -1362,10 +1363,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
                         wR[n] = w.y;
                     }
                     if constexpr (NPH) {
-                        // FP32 reconstruction, FP64 limiter (WENO5; WENO5B bounds its face values instead) and
-                        // Riemann solver
+                        // FP32 reconstruction, FP64 limiter and Riemann solver
                         const int b = T::base(d, t), h = T::halo(d, t), sd = T::stride(d);
-                        nphase_mixed_face<M, SCHEME == 5>(
+                        nphase_mixed_face<M, LIMIT>(
                             F, fnc, cm, wL, wR, prim + T::cell(b, sd, h, fd - 1), prim + T::cell(b, sd, h, fd), CSTR, dxd,
                             a.e, d, a.id_k, a.riemann == 2, [&](const double* UL, const double* UR) {
                                 riemann<M>(a.riemann, F, fnc, cm, UL, UR, a.e, d, a.id_k, err);
@@ -1412,7 +1412,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& a, int tile, double*
             if (a.mode == kModeCmax) {
                 // wave speeds only: with one halo set resident, the next direction's conversion rewrites the planes
                 // that the limiter of this flux pass reads
-                if constexpr (NHS != D) __syncthreads();
+                if constexpr (LIMIT && NHS != D) __syncthreads();
                 continue;
             }
             __syncthreads();
